@@ -91,3 +91,23 @@ def test_symmetric_product_computes_upper_tiles_and_mirrors(n, k):
     sym3 = ops.gemm(xt, xt, a_t=True, b_t=True, symmetric=True)
     torch.testing.assert_close(sym3.float(), ref, rtol=2e-2, atol=2e-2 * float(ref.abs().max()) / 16)
     ops.check_status()
+
+
+@pytest.mark.parametrize("n", [264, 520, 1000])
+@pytest.mark.parametrize("c_dtype,shift", [(torch.bfloat16, 0), (torch.bfloat16, 3), (torch.float32, 0), (torch.float32, 1)])
+def test_symmetric_product_with_ragged_edge_and_any_addend(n, c_dtype, shift):
+    """Sizes that end inside a tile, addends that start off a 16-byte boundary (element-wise loads) or on one: the mirrored
+    half is exact and nothing outside [n, n] is written. Error bound: one bf16 rounding of the result (2^-8 of each
+    element) and fp32 sums."""
+    torch.manual_seed(1)
+    dev = torch.device("cuda")
+    x = torch.randn(n, 192, device=dev).bfloat16()
+    c = torch.randn(n, n + 8, device=dev).to(c_dtype)
+    c[:, shift:shift + n] = torch.triu(c[:, shift:shift + n]) + torch.triu(c[:, shift:shift + n], 1).t()
+    c = c[:, shift:shift + n]
+    out = torch.full((n, n + 8), 7.0, device=dev, dtype=torch.bfloat16)
+    ops.gemm(x, x, out=out[:, :n], c=c, alpha=0.5, beta=-1.5, symmetric=True)
+    ref = 0.5 * (x.double() @ x.double().t()) - 1.5 * c.double()
+    assert torch.equal(out[:, :n], out[:, :n].t()) and bool((out[:, n:] == 7.0).all())
+    assert bool(((out[:, :n].double() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-4).all())
+    ops.check_status()
