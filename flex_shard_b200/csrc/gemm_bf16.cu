@@ -46,6 +46,7 @@ struct GemmArgs {
   int c_fp32;
   float alpha, beta;
   int accumulate;
+  int batch;          // two-SM kernel, batched form: equal matrices stacked back to back in A, B, C and D
   int upper_only;     // two-SM kernel, M == N: compute only the 256x256 tiles on or above the diagonal and mirror them
   // When d_block_rows > 0, D is cut into blocks of that many rows and block i starts at
   // element offset i * d_block_stride (the [world, rows/world, N] rows of a reduce-scatter
@@ -689,6 +690,20 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr,
+                                                 int32_t c0, int32_t c1, int32_t c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+template <bool BATCH>
+__device__ __forceinline__ void load_tile_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr,
+                                               int32_t c0, int32_t c1, int32_t e) {
+  if constexpr (BATCH) tma_load_3d_pair(smem_dst, map, bar_cluster_addr, c0, c1, e);
+  else tma_load_2d_pair(smem_dst, map, bar_cluster_addr, c0, c1);
+}
 __device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                               uint32_t accumulate) {
   asm volatile(
@@ -722,6 +737,33 @@ __device__ __forceinline__ void upper_tile_coords(int t, int T, int& tm, int& tn
   tn = tm + t;
 }
 
+// Which 256x256 tile of which matrix a pair works on.
+struct PairTile {
+  int tm2, tn, e;
+};
+template <bool BATCH>
+__device__ __forceinline__ PairTile pair_tile(const GemmArgs& args, int tile, int tiles_m, int tiles_n, int per_matrix,
+                                              bool spread) {
+  PairTile t;
+  t.e = 0;
+  if (BATCH) {
+    t.e = tile / per_matrix;
+    tile -= t.e * per_matrix;
+  }
+  if (args.upper_only) {
+    upper_tile_coords(tile, tiles_m, t.tm2, t.tn);
+  } else {
+    tile_coords(tile, tiles_m, tiles_n, t.tm2, t.tn);
+    if (spread) t.tm2 = spread_over_row_blocks(t.tm2, tiles_m, args.d_peer_n);
+  }
+  return t;
+}
+
+// BATCH: args.batch equal matrices per operand, addressed through 3-D tensor maps, so the edge of every matrix is
+// filled with zeros and M, N, K need not be multiples of a tile. All matrices share one persistent grid: a stack of
+// small products (attention heads, experts) fills the SMs that a launch per matrix would leave idle, and each product
+// of a stack costs one launch.
+template <bool BATCH>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                      const GemmArgs args) {
@@ -741,7 +783,8 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   const uint32_t rank = cluster_ctarank();
   const int tiles_m = (args.M + 2 * BM - 1) / (2 * BM);   // 256-row tiles
   const int tiles_n = (args.N + BN - 1) / BN;
-  const int num_tiles = args.upper_only ? tiles_m * (tiles_m + 1) / 2 : tiles_m * tiles_n;
+  const int per_matrix = args.upper_only ? tiles_m * (tiles_m + 1) / 2 : tiles_m * tiles_n;
+  const int num_tiles = BATCH ? per_matrix * args.batch : per_matrix;
   const int num_kb = (args.K + BK - 1) / BK;
   const int tile0 = static_cast<int>(blockIdx.x >> 1);
   const int tile_step = static_cast<int>(gridDim.x >> 1);
@@ -780,15 +823,9 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       uint32_t it = 0;
       bool ok = true;
       for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
-        int tm2, tn;
-        if (args.upper_only) {
-          upper_tile_coords(tile, tiles_m, tm2, tn);
-        } else {
-          tile_coords(tile, tiles_m, tiles_n, tm2, tn);
-          if (spread) tm2 = spread_over_row_blocks(tm2, tiles_m, args.d_peer_n);
-        }
-        const int m0 = tm2 * 2 * BM + static_cast<int>(rank) * BM;
-        const int n0 = tn * BN + static_cast<int>(rank) * BN_HALF;
+        const PairTile pt = pair_tile<BATCH>(args, tile, tiles_m, tiles_n, per_matrix, spread);
+        const int m0 = pt.tm2 * 2 * BM + static_cast<int>(rank) * BM;
+        const int n0 = pt.tn * BN + static_cast<int>(rank) * BN_HALF;
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % STAGES2;
           const uint32_t ph = (it / STAGES2) & 1;
@@ -804,16 +841,17 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
           if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * STAGE2_BYTES);   // the bytes of both CTAs
           const int k0 = kb * BK;
           if (!args.a_mn) {
-            tma_load_2d_pair(sa, &map_a, full0, k0, m0);
+            load_tile_pair<BATCH>(sa, &map_a, full0, k0, m0, pt.e);
           } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * 8192, &map_a, full0, m0 + 64 * j, k0);
+            for (int j = 0; j < BM / 64; ++j) load_tile_pair<BATCH>(sa + j * 8192, &map_a, full0, m0 + 64 * j, k0, pt.e);
           }
           if (!args.b_mn) {
-            tma_load_2d_pair(sb, &map_b, full0, k0, n0);
+            load_tile_pair<BATCH>(sb, &map_b, full0, k0, n0, pt.e);
           } else {
 #pragma unroll
-            for (int j = 0; j < BN_HALF / 64; ++j) tma_load_2d_pair(sb + j * 8192, &map_b, full0, n0 + 64 * j, k0);
+            for (int j = 0; j < BN_HALF / 64; ++j)
+              load_tile_pair<BATCH>(sb + j * 8192, &map_b, full0, n0 + 64 * j, k0, pt.e);
           }
         }
       }
@@ -880,14 +918,8 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const int quarter = warp & 3;
     uint32_t local_tile = 0;
     for (int tile = tile0; tile < num_tiles; tile += tile_step) {
-      int tm2, tn;
-      if (args.upper_only) {
-        upper_tile_coords(tile, tiles_m, tm2, tn);
-      } else {
-        tile_coords(tile, tiles_m, tiles_n, tm2, tn);
-        if (spread) tm2 = spread_over_row_blocks(tm2, tiles_m, args.d_peer_n);
-      }
-      const int tm = tm2 * 2 + static_cast<int>(rank);
+      const PairTile pt = pair_tile<BATCH>(args, tile, tiles_m, tiles_n, per_matrix, spread);
+      const int tm = pt.tm2 * 2 + static_cast<int>(rank);
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_ph = (local_tile >> 1) & 1;
       ++local_tile;
@@ -899,9 +931,10 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         break;
       }
       tc_fence_after();
-      store_tile(args, 0, tm, tn, tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16),
+      store_tile(args, BATCH ? static_cast<long long>(pt.e) * args.M : 0, tm, pt.tn,
+                 tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16),
                  reinterpret_cast<float*>(smem + STAGES2 * STAGE2_BYTES + 256) + (warp - 2) * 32 * 33, quarter, lane,
-                 args.upper_only && tm2 != tn);
+                 args.upper_only && pt.tm2 != pt.tn);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
@@ -977,6 +1010,28 @@ int fsb_make_tmap_2d(CUtensorMap* map, const void* base, CUtensorMapDataType dty
   return FSB_OK;
 }
 
+// bf16 stack [count, rows, cols] of row-major matrices (row stride ld, matrices back to back); box = one matrix's
+// [box_rows, box_cols], 128-byte swizzle.
+static int make_tmap_stack_bf16(CUtensorMap* map, const void* base, uint64_t count, uint64_t rows, uint64_t cols,
+                                uint64_t ld, uint32_t box_rows, uint32_t box_cols) {
+  FsbEncodeTiledFn enc = fsb_get_encode_tiled();
+  if (enc == nullptr) return FSB_ERR_TMA_ENCODE;
+  static thread_local bool ctx_bound = false;   // see fsb_make_tmap_2d
+  if (!ctx_bound) {
+    cudaFree(nullptr);
+    ctx_bound = true;
+  }
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (ld * 2) % 16 != 0) return FSB_ERR_BAD_ARG;
+  cuuint64_t dims[3] = {cols, rows, count};
+  cuuint64_t strides[2] = {ld * 2, rows * ld * 2};
+  cuuint32_t box[3] = {box_cols, box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? FSB_OK : FSB_ERR_TMA_ENCODE;
+}
+
 int fsb_make_tmap_2d_plain(CUtensorMap* map, const void* base, CUtensorMapDataType dtype,
                            int elem_size, uint64_t rows, uint64_t cols, uint64_t ld,
                            uint32_t box_rows, uint32_t box_cols) {
@@ -1006,18 +1061,14 @@ int fsb_make_tmap_2d_plain(CUtensorMap* map, const void* base, CUtensorMapDataTy
 static int g_use_pairs_value();
 static inline bool g_use_pairs_fwd() { return g_use_pairs_value() != 0; }
 
-static int gemm_pair_launch(const void* a, const void* b, void* d, const void* c, int M, int N, int K,
-                            long long lda, long long ldb, long long ldd, long long ldc, int a_mn, int b_mn,
-                            int d_fp32, int c_fp32, float alpha, float beta, int accumulate,
-                            long long d_block_rows, long long d_block_stride, const unsigned long long* d_peer,
-                            int d_peer_n, int* status, cudaStream_t stream, int upper_only = 0) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return FSB_ERR_BAD_ARG;
+// Co-resident clusters of the two-SM kernels on device `dev` (-1: unusable); sets their shared-memory limits once.
+static int pair_clusters(int dev) {
   if (g_pair_clusters[dev] == 0) {
-    g_pair_clusters[dev] = -1;
-    if (cudaFuncSetAttribute(gemm_bf16_2sm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES) ==
-        cudaSuccess) {
+    int found = -1;
+    if (cudaFuncSetAttribute(gemm_bf16_2sm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES) ==
+            cudaSuccess &&
+        cudaFuncSetAttribute(gemm_bf16_2sm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES) ==
+            cudaSuccess) {
       cudaLaunchConfig_t cfg{};
       cfg.gridDim = dim3(2, 1, 1);
       cfg.blockDim = dim3(NUM_THREADS, 1, 1);
@@ -1030,11 +1081,23 @@ static int gemm_pair_launch(const void* a, const void* b, void* d, const void* c
       cfg.attrs = &at;
       cfg.numAttrs = 1;
       int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, gemm_bf16_2sm_kernel, &cfg) == cudaSuccess && n > 0)
-        g_pair_clusters[dev] = n;
+      if (cudaOccupancyMaxActiveClusters(&n, gemm_bf16_2sm_kernel<false>, &cfg) == cudaSuccess && n > 0) found = n;
     }
     cudaGetLastError();
+    g_pair_clusters[dev] = found;
   }
+  return g_pair_clusters[dev];
+}
+
+static int gemm_pair_launch(const void* a, const void* b, void* d, const void* c, int M, int N, int K,
+                            long long lda, long long ldb, long long ldd, long long ldc, int a_mn, int b_mn,
+                            int d_fp32, int c_fp32, float alpha, float beta, int accumulate,
+                            long long d_block_rows, long long d_block_stride, const unsigned long long* d_peer,
+                            int d_peer_n, int* status, cudaStream_t stream, int upper_only = 0) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return FSB_ERR_BAD_ARG;
+  pair_clusters(dev);
   if (g_pair_clusters[dev] < 0) return FSB_ERR_TOO_LARGE;
   CUtensorMap map_a, map_b;
   int rc;
@@ -1062,7 +1125,46 @@ static int gemm_pair_launch(const void* a, const void* b, void* d, const void* c
     args.upper_only = 1;
   }
   const int clusters = tiles < g_pair_clusters[dev] ? static_cast<int>(tiles) : g_pair_clusters[dev];
-  gemm_bf16_2sm_kernel<<<2 * clusters, NUM_THREADS, SMEM2_BYTES, stream>>>(map_a, map_b, args);
+  gemm_bf16_2sm_kernel<false><<<2 * clusters, NUM_THREADS, SMEM2_BYTES, stream>>>(map_a, map_b, args);
+  return cudaGetLastError() == cudaSuccess ? FSB_OK : FSB_ERR_LAUNCH;
+}
+
+// D_e = alpha * A_e . B_e^T + beta * C_e for `count` equal matrices, each operand a stack of row-major bf16 matrices back
+// to back (A [count, M, K] or, a_mn, [count, K, M]; B likewise; C and D [count, M, N], all rows packed). Contiguous
+// dimensions must be multiples of 8. symmetric: every D_e is symmetric (M == N); only its tiles on or above the diagonal
+// are computed, and mirrored. Returns FSB_ERR_TOO_LARGE where SM pairs cannot be used.
+//
+// Bound by the tensor cores for stacks of expert matrices, by latency for a stack of attention heads (a 192 x 1536
+// matrix is a single tile, so one grid takes the whole stack). A Muon step over 64 experts of 2816 x 2048 and of
+// 2048 x 1408, 64 attention-head matrices and the ten single matrices of two blocks: 64.7 ms with the one-SM grouped
+// kernel (full products, heads one at a time), 28.8 ms here, 18.4 ms of them in this kernel (about 1 180 TFLOP/s of
+// executed products).
+FSB_API int fsb_gemm_bf16_batched(const void* a, const void* b, void* d, const void* c, int count, int M, int N, int K,
+                                  int a_mn, int b_mn, float alpha, float beta, int symmetric, int* status,
+                                  cudaStream_t stream) {
+  if (count <= 0 || M <= 0 || N <= 0 || K <= 0 || (symmetric && M != N)) return FSB_ERR_BAD_ARG;
+  if ((a_mn ? M : K) % 8 != 0 || (b_mn ? N : K) % 8 != 0 || N % 8 != 0) return FSB_ERR_BAD_ARG;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return FSB_ERR_BAD_ARG;
+  if (pair_clusters(dev) < 0) return FSB_ERR_TOO_LARGE;
+  const long long tm = (M + 2 * BM - 1) / (2 * BM), tn = (N + BN - 1) / BN;
+  const int upper = symmetric && tm > 1;
+  const long long tiles = (upper ? tm * (tm + 1) / 2 : tm * tn) * count;
+  if (tiles >= (1ll << 31)) return FSB_ERR_TOO_LARGE;
+  CUtensorMap map_a, map_b;
+  int rc = a_mn ? make_tmap_stack_bf16(&map_a, a, count, K, M, M, BK, 64) : make_tmap_stack_bf16(&map_a, a, count, M, K, K, BM, BK);
+  if (rc != FSB_OK) return rc;
+  rc = b_mn ? make_tmap_stack_bf16(&map_b, b, count, K, N, N, BK, 64) : make_tmap_stack_bf16(&map_b, b, count, N, K, K, BN_HALF, BK);
+  if (rc != FSB_OK) return rc;
+  GemmArgs args{};
+  args.M = M; args.N = N; args.K = K; args.a_mn = a_mn; args.b_mn = b_mn; args.batch = count;
+  args.d = d; args.ldd = N; args.c = c; args.ldc = N;
+  args.alpha = alpha; args.beta = c != nullptr ? beta : 0.f;
+  args.upper_only = upper;
+  args.status = status;
+  const int clusters = tiles < g_pair_clusters[dev] ? static_cast<int>(tiles) : g_pair_clusters[dev];
+  gemm_bf16_2sm_kernel<true><<<2 * clusters, NUM_THREADS, SMEM2_BYTES, stream>>>(map_a, map_b, args);
   return cudaGetLastError() == cudaSuccess ? FSB_OK : FSB_ERR_LAUNCH;
 }
 
@@ -1083,31 +1185,11 @@ FSB_API int fsb_gemm_bf16(const void* a, const void* b, void* d, const void* c, 
 //           number of valid m-tiles (device memory: no host synchronisation), max_mtiles bounds it.
 //   mode 2: D[E, M, N] = sum over each expert's rows of A[r, :M]^T B[r, :N] (A, B row-major
 //           [R, M] / [R, N]); group_offs is the int[E+1] array of padded row offsets.
-FSB_API int fsb_gemm_bf16_grouped_ex(const void* a, const void* b, void* d, int mode, int num_groups, int M,
-                                     int N, int K, long long lda, long long ldb, long long ldd, int b_mn,
-                                     int d_fp32, int accumulate, const int* tile_expert,
-                                     const int* num_mtiles, const int* group_offs, int max_rows,
-                                     const void* c, long long ldc, int c_fp32, float alpha, float beta,
-                                     int* status, cudaStream_t stream);
-
 FSB_API int fsb_gemm_bf16_grouped(const void* a, const void* b, void* d, int mode, int num_groups, int M,
                                   int N, int K, long long lda, long long ldb, long long ldd, int b_mn,
                                   int d_fp32, int accumulate, const int* tile_expert,
                                   const int* num_mtiles, const int* group_offs, int max_rows,
                                   int* status, cudaStream_t stream) {
-  return fsb_gemm_bf16_grouped_ex(a, b, d, mode, num_groups, M, N, K, lda, ldb, ldd, b_mn, d_fp32, accumulate,
-                                  tile_expert, num_mtiles, group_offs, max_rows, nullptr, 0, 0, 1.f, 0.f, status,
-                                  stream);
-}
-
-// The same with the dense GEMM's epilogue: D = alpha * product + beta * C, where C has D's layout
-// ([R, N] rows for mode 1, [E, M, N] for mode 2).
-FSB_API int fsb_gemm_bf16_grouped_ex(const void* a, const void* b, void* d, int mode, int num_groups, int M,
-                                     int N, int K, long long lda, long long ldb, long long ldd, int b_mn,
-                                     int d_fp32, int accumulate, const int* tile_expert,
-                                     const int* num_mtiles, const int* group_offs, int max_rows,
-                                     const void* c, long long ldc, int c_fp32, float alpha, float beta,
-                                     int* status, cudaStream_t stream) {
   if (mode != 1 && mode != 2) return FSB_ERR_BAD_ARG;
   CUtensorMap map_a, map_b;
   int rc;
@@ -1131,8 +1213,7 @@ FSB_API int fsb_gemm_bf16_grouped_ex(const void* a, const void* b, void* d, int 
     if (rc != FSB_OK) return rc;
     args.M = M; args.N = N; args.K = max_rows; args.a_mn = 1; args.b_mn = 1;
   }
-  args.d = d; args.ldd = ldd; args.d_fp32 = d_fp32; args.alpha = alpha; args.beta = c != nullptr ? beta : 0.f;
-  args.c = c; args.ldc = ldc; args.c_fp32 = c_fp32;
+  args.d = d; args.ldd = ldd; args.d_fp32 = d_fp32; args.alpha = 1.f;
   args.accumulate = accumulate; args.group_mode = mode; args.num_groups = num_groups;
   args.tile_expert = tile_expert; args.num_mtiles = num_mtiles; args.group_offs = group_offs;
   args.status = status;

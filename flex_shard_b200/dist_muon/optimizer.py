@@ -299,14 +299,14 @@ class DistMuon(torch.optim.Optimizer):
     def _stack_step(self, p3, g3, m3, group) -> bool:
         """One step for a stack ``[n, rows, cols]`` of equal matrices in one go (momentum over the whole stack,
         per-matrix normalisation, the batched Newton-Schulz iteration, one update): used when the batched
-        iteration applies (CUDA, dimensions multiples of 128), else the caller loops over the matrices."""
-        from ..ops.newton_schulz import batched_ns_supported, muon_momentum_direction_, newton_schulz
+        iteration applies (CUDA, dimensions multiples of 8), else the caller loops over the matrices."""
+        from ..ops.newton_schulz import batched_ns_supported
 
         if not (p3.dim() == 3 and p3.is_contiguous() and m3.is_contiguous() and batched_ns_supported(p3)):
             return False
-        u = muon_momentum_direction_(m3, g3.contiguous(), group["momentum"], group["nesterov"])
-        x = newton_schulz(u, group["ns_steps"], group["ns_coefficients"], group["eps"])
-        muon_apply_(p3, x.contiguous(), float(group["lr"]), group["weight_decay"],
+        x = muon_direction_(m3, g3.contiguous(), group["momentum"], group["nesterov"], group["ns_steps"],
+                            group["ns_coefficients"], group["eps"])
+        muon_apply_(p3, x, float(group["lr"]), group["weight_decay"],
                     lr_ratio(group["adjust_lr_fn"], p3.shape[1], p3.shape[2]))
         return True
 

@@ -31,17 +31,20 @@ def _ensure():
     if not _declared:
         c = ctypes
         vp, i32, i64, f32 = c.c_void_p, c.c_int, c.c_longlong, c.c_float
-        _lib.declare("fsb_muon_prepare", [vp, vp, i32, vp, vp, i64, f32, i32, vp])
-        _lib.declare("fsb_muon_scale", [vp, vp, i64, f32, vp])
+        _lib.declare("fsb_muon_prepare", [vp, vp, i32, vp, vp, i64, i32, f32, i32, vp])
+        _lib.declare("fsb_muon_scale", [vp, vp, i32, i64, i32, f32, vp])
         _lib.declare("fsb_muon_update", [vp, i32, vp, i64, f32, f32, vp])
-        _lib.declare("fsb_muon_workspace_floats", [])
+        _lib.declare("fsb_muon_workspace_floats", [i64, i32])
+        _lib.declare("fsb_gemm_bf16_batched", [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, f32, i32, vp, vp])
         _declared = True
 
 
-def _workspace(device) -> torch.Tensor:
-    """Zeroed scratch of the prepare kernel: [0] receives the sum of squares, the rest holds the per-block
-    partial sums, which the last block adds in index order (the same bits on every run)."""
-    return torch.zeros(_lib.load().fsb_muon_workspace_floats(), dtype=torch.float32, device=device)
+def _workspace(device, n: int, count: int = 1) -> torch.Tensor:
+    """Zeroed scratch ``[count, floats]`` of the prepare kernel for ``count`` matrices of ``n`` elements: [m, 0] receives
+    matrix m's sum of squares, the rest of its row holds the per-block partial sums, which the matrix's last block adds
+    in index order (the same bits on every run)."""
+    floats = _lib.load().fsb_muon_workspace_floats(n, count)
+    return torch.zeros(count, floats // count, dtype=torch.float32, device=device)
 
 
 def ns_iterations(x: torch.Tensor, steps: int = 5, coeffs=NS_COEFFS) -> torch.Tensor:
@@ -66,74 +69,44 @@ def ns_iterations(x: torch.Tensor, steps: int = 5, coeffs=NS_COEFFS) -> torch.Te
     return x
 
 
-_batch_tables: dict = {}
-
-
-def _tables(E: int, rows: int, device):
-    """Grouped-GEMM tables of ``E`` equal groups of ``rows`` rows (``rows`` a multiple of 128): the group of every
-    128-row tile, the tile count and the group offsets, as device tensors."""
-    key = (E, rows, device)
-    t = _batch_tables.get(key)
-    if t is None:
-        tile_group = torch.arange(E, dtype=torch.int32).repeat_interleave(rows // 128).to(device)
-        count = torch.tensor([E * rows // 128], dtype=torch.int32, device=device)
-        offs = (torch.arange(E + 1, dtype=torch.int64) * rows).to(torch.int32).to(device)
-        t = _batch_tables[key] = (tile_group, count, offs)
-        if len(_batch_tables) > 256:
-            _batch_tables.pop(next(iter(_batch_tables)))
-    return t
-
-
-def _grouped(mode, a, b, out, E, M, N, K, b_mn, tables, max_rows, c=None, alpha=1.0, beta=0.0):
-    lib = _lib.load()
-    fn = lib.fsb_gemm_bf16_grouped_ex
-    if not getattr(fn, "_fsb_declared", False):
-        cc = ctypes
-        vp, i32, i64, f32 = cc.c_void_p, cc.c_int, cc.c_longlong, cc.c_float
-        fn.argtypes = [vp, vp, vp, i32, i32, i32, i32, i32, i64, i64, i64, i32, i32, i32, vp, vp, vp, i32,
-                       vp, i64, i32, f32, f32, vp, vp]
-        fn.restype = cc.c_int
-        fn._fsb_declared = True
-    tile_group, count, offs = tables
-    rc = fn(a.data_ptr(), b.data_ptr(), out.data_ptr(), mode, E, M, N, K, a.stride(0), b.stride(0), out.stride(-2),
-            int(b_mn), 0, 0, tile_group.data_ptr(), count.data_ptr(), offs.data_ptr(), max_rows,
-            c.data_ptr() if c is not None else None, c.stride(-2) if c is not None else 0, 0, alpha, beta,
-            _lib.status_word(a.device).data_ptr(), _lib.stream_ptr(a.device))
-    _lib.check(rc, "fsb_gemm_bf16_grouped_ex")
+def _batched(a, b, out, M, N, K, *, a_t=False, b_t=False, c=None, alpha=1.0, beta=0.0, symmetric=False):
+    """One product for every matrix of contiguous stacks: ``out[e] = alpha * A[e] @ B[e]^T + beta * c[e]``."""
+    _ensure()
+    rc = _lib.load().fsb_gemm_bf16_batched(
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), c.data_ptr() if c is not None else None, a.shape[0], M, N, K,
+        int(a_t), int(b_t), alpha, beta, int(symmetric), _lib.status_word(a.device).data_ptr(), _lib.stream_ptr(a.device))
+    _lib.check(rc, "fsb_gemm_bf16_batched")
     count_launch()
 
 
 def batched_ns_supported(x: torch.Tensor) -> bool:
-    """Stacks of equal matrices whose dimensions are multiples of 128 run every product of an iteration as one
-    grouped launch over the whole stack."""
-    return (x.is_cuda and x.dim() == 3 and x.shape[0] > 1 and x.shape[1] % 128 == 0 and x.shape[2] % 128 == 0)
+    """Stacks of equal matrices whose dimensions are multiples of 8 (16-byte rows, which the copy engine needs) run every
+    product of an iteration as one launch over the whole stack."""
+    return (x.is_cuda and x.dim() == 3 and 1 < x.shape[0] <= 65535 and x.shape[1] % 8 == 0 and x.shape[2] % 8 == 0
+            and x.numel() > 0)
 
 
 def ns_iterations_batched(x: torch.Tensor, steps: int = 5, coeffs=NS_COEFFS) -> torch.Tensor:
-    """The iteration on a stack ``[E, rows, cols]`` of normalised bf16 matrices: three grouped GEMM launches per
-    step for all ``E`` matrices (per-head and per-expert matrices are small; one launch each would leave most of
-    the GPU idle and pay 15 launches per matrix).  Same arithmetic per matrix as ``ns_iterations``."""
+    """The iteration on a stack ``[E, rows, cols]`` of normalised bf16 matrices: three GEMM launches per step for all
+    ``E`` matrices (per-head and per-expert matrices are small; one launch each would leave most of the GPU idle and pay
+    15 launches per matrix).  Same arithmetic per matrix as ``ns_iterations``."""
     a, b, c = coeffs
     E, rows, cols = x.shape
     wide = rows <= cols
     s = min(rows, cols)
     x = x.contiguous()
-    dev = x.device
-    A = torch.empty(E, s, s, dtype=x.dtype, device=dev)
-    B = torch.empty(E, s, s, dtype=x.dtype, device=dev)
+    A = torch.empty(E, s, s, dtype=x.dtype, device=x.device)
+    B = torch.empty_like(A)
     nxt = torch.empty_like(x)
-    t_s, t_rows = _tables(E, s, dev), _tables(E, rows, dev)
-    A2, B2 = A.view(E * s, s), B.view(E * s, s)
     for _ in range(steps):
-        x2, n2 = x.view(E * rows, cols), nxt.view(E * rows, cols)
         if wide:
-            _grouped(1, x2, x2, A2, E, E * s, s, cols, False, t_s, E * s)                      # A = X X^T
-            _grouped(1, A2, A2, B2, E, E * s, s, s, False, t_s, E * s, c=A2, alpha=c, beta=b)  # B = b A + c A A
-            _grouped(1, B2, x2, n2, E, E * s, cols, s, True, t_s, E * s, c=x2, alpha=1.0, beta=a)   # X = a X + B X
+            _batched(x, x, A, s, s, cols, symmetric=True)                                # A = X X^T
+            _batched(A, A, B, s, s, s, c=A, alpha=c, beta=b, symmetric=True)             # B = b A + c A A
+            _batched(B, x, nxt, s, cols, s, b_t=True, c=x, beta=a)                       # X = a X + B X
         else:
-            _grouped(2, x2, x2, A, E, s, s, E * rows, True, t_rows, E * rows)                   # A = X^T X
-            _grouped(1, A2, A2, B2, E, E * s, s, s, False, t_s, E * s, c=A2, alpha=c, beta=b)
-            _grouped(1, x2, B2, n2, E, E * rows, s, s, False, t_rows, E * rows, c=x2, alpha=1.0, beta=a)  # X = a X + X B
+            _batched(x, x, A, s, s, rows, a_t=True, b_t=True, symmetric=True)            # A = X^T X
+            _batched(A, A, B, s, s, s, c=A, alpha=c, beta=b, symmetric=True)
+            _batched(x, B, nxt, rows, s, s, c=x, beta=a)                                 # X = a X + X B
         x, nxt = nxt, x
     return x
 
@@ -180,35 +153,45 @@ def _normalise_cuda(x: torch.Tensor, eps: float) -> torch.Tensor:
     _ensure()
     x = x.contiguous().clone()
     ss = (x.float() ** 2).sum().reshape(1)
-    rc = _lib.load().fsb_muon_scale(x.data_ptr(), ss.data_ptr(), x.numel(), eps, _lib.stream_ptr(x.device))
+    rc = _lib.load().fsb_muon_scale(x.data_ptr(), ss.data_ptr(), 1, x.numel(), 1, eps, _lib.stream_ptr(x.device))
     _lib.check(rc, "fsb_muon_scale")
     count_launch()
     return x
 
 
+def _prepare(momentum, grad, mu, nesterov, count):
+    """Momentum update in place and the bf16 direction before orthogonalisation, with the squared norms of its ``count``
+    equal matrices."""
+    _ensure()
+    g = grad.contiguous()
+    assert momentum.is_contiguous() and momentum.dtype == torch.float32 and momentum.shape == grad.shape
+    n = g.numel() // count
+    u = torch.empty(g.shape, dtype=torch.bfloat16, device=g.device)
+    ws = _workspace(g.device, n, count)
+    rc = _lib.load().fsb_muon_prepare(momentum.data_ptr(), g.data_ptr(), int(g.dtype == torch.float32), u.data_ptr(),
+                                      ws.data_ptr(), n, count, mu, int(nesterov), _lib.stream_ptr(g.device))
+    _lib.check(rc, "fsb_muon_prepare")
+    count_launch()
+    return u, ws
+
+
 def muon_direction_(momentum: torch.Tensor, grad: torch.Tensor, mu: float, nesterov: bool, steps: int,
                     coeffs=NS_COEFFS, eps: float = 1e-7) -> torch.Tensor:
     """Momentum update (in place, fp32) + Nesterov + normalise + Newton-Schulz; returns the bf16
-    direction with the shape of ``grad`` (2-D)."""
-    assert grad.dim() == 2 and momentum.shape == grad.shape
+    direction with the shape of ``grad`` (2-D, or on CUDA a stack ``[n, rows, cols]`` of equal matrices that
+    ``batched_ns_supported`` accepts)."""
+    assert momentum.shape == grad.shape and (grad.dim() == 2 or batched_ns_supported(grad))
     if not grad.is_cuda:
         momentum.lerp_(grad.float(), 1 - mu)
         u = grad.float().lerp(momentum, mu) if nesterov else momentum
         return _newton_schulz_cpu(u, steps, coeffs, eps)
-    _ensure()
-    lib = _lib.load()
-    g = grad.contiguous()
-    assert momentum.is_contiguous() and momentum.dtype == torch.float32
-    u = torch.empty(g.shape, dtype=torch.bfloat16, device=g.device)
-    ss = _workspace(g.device)
-    s = _lib.stream_ptr(g.device)
-    rc = lib.fsb_muon_prepare(momentum.data_ptr(), g.data_ptr(), int(g.dtype == torch.float32), u.data_ptr(),
-                              ss.data_ptr(), g.numel(), mu, int(nesterov), s)
-    _lib.check(rc, "fsb_muon_prepare")
-    rc = lib.fsb_muon_scale(u.data_ptr(), ss.data_ptr(), u.numel(), eps, s)
+    count = grad.shape[0] if grad.dim() == 3 else 1
+    u, ws = _prepare(momentum, grad, mu, nesterov, count)
+    rc = _lib.load().fsb_muon_scale(u.data_ptr(), ws.data_ptr(), ws.shape[1], u.numel() // count, count, eps,
+                                    _lib.stream_ptr(u.device))
     _lib.check(rc, "fsb_muon_scale")
-    count_launch(2)
-    return ns_iterations(u, steps, coeffs)
+    count_launch()
+    return (ns_iterations_batched if grad.dim() == 3 else ns_iterations)(u, steps, coeffs)
 
 
 def muon_momentum_direction_(momentum: torch.Tensor, grad: torch.Tensor, mu: float, nesterov: bool) -> torch.Tensor:
@@ -219,16 +202,7 @@ def muon_momentum_direction_(momentum: torch.Tensor, grad: torch.Tensor, mu: flo
         momentum.lerp_(grad.float(), 1 - mu)
         u = grad.float().lerp(momentum, mu) if nesterov else momentum
         return u.to(torch.bfloat16)
-    _ensure()
-    g = grad.contiguous()
-    assert momentum.is_contiguous()
-    u = torch.empty(g.shape, dtype=torch.bfloat16, device=g.device)
-    ss = _workspace(g.device)
-    rc = _lib.load().fsb_muon_prepare(momentum.data_ptr(), g.data_ptr(), int(g.dtype == torch.float32), u.data_ptr(),
-                                      ss.data_ptr(), g.numel(), mu, int(nesterov), _lib.stream_ptr(g.device))
-    _lib.check(rc, "fsb_muon_prepare")
-    count_launch()
-    return u
+    return _prepare(momentum, grad, mu, nesterov, 1)[0]
 
 
 def muon_apply_(param: torch.Tensor, direction: torch.Tensor, lr: float, weight_decay: float, ratio: float):

@@ -119,3 +119,56 @@ def test_dist_muon_steps_a_stack_of_equal_matrices_in_one_go():
         torch.testing.assert_close(stacked.detach()[i], p.detach(), rtol=0, atol=2e-3)
     assert launches[0] * 3 < launches[1]            # 1 + 15 + 1 launches (plus normalisation) against 6 x 18
     ops.check_status()
+
+
+@pytest.mark.parametrize("E,rows,cols", [(5, 192, 1536), (3, 40, 72), (4, 520, 264), (2, 1000, 8), (70, 8, 128), (2, 256, 512)])
+def test_batched_products_of_any_size_stay_inside_their_matrix(E, rows, cols):
+    """Every product form of the iteration on stacks whose matrices end inside a tile. Bound: one bf16 rounding of the
+    result (2^-8 of each element) and fp32 sums over at most 1536 terms of unit variance."""
+    torch.manual_seed(8)
+    x = torch.randn(E, rows, cols, device="cuda").bfloat16()
+    xd = x.double()
+    s = min(rows, cols)
+    gram = xd @ xd.mT if rows <= cols else xd.mT @ xd
+
+    def check(out, ref):
+        assert bool(((out.double() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-3).all())
+
+    buf = torch.full((E + 1, s, s), 7.0, device="cuda", dtype=torch.bfloat16)
+    A = buf[:E]
+    if rows <= cols:
+        ns._batched(x, x, A, s, s, cols, symmetric=True)
+    else:
+        ns._batched(x, x, A, s, s, rows, a_t=True, b_t=True, symmetric=True)
+    check(A, gram)
+    assert torch.equal(A, A.mT) and bool((buf[E] == 7.0).all())
+    A = (A.float() / s).bfloat16()
+    B = torch.empty_like(A)
+    ns._batched(A, A, B, s, s, s, c=A, alpha=0.5, beta=-1.5, symmetric=True)
+    check(B, 0.5 * (A.double() @ A.double()) - 1.5 * A.double())
+    assert torch.equal(B, B.mT)
+    nxt = torch.empty_like(x)
+    if rows <= cols:
+        ns._batched(B, x, nxt, s, cols, s, b_t=True, c=x, beta=2.0)
+        check(nxt, B.double() @ xd + 2.0 * xd)
+    else:
+        ns._batched(x, B, nxt, rows, s, s, c=x, beta=2.0)
+        check(nxt, xd @ B.double() + 2.0 * xd)
+    ops.check_status()
+
+
+@pytest.mark.parametrize("E,rows,cols", [(3, 40, 72), (2, 5, 9), (1, 300, 700)])
+def test_prepare_and_scale_of_a_stack_match_the_matrices_alone(E, rows, cols):
+    """One launch over a stack gives the bits of one launch per matrix, sums of squares included up to their order
+    (fp32 sums of at most 210 000 terms)."""
+    torch.manual_seed(9)
+    g = torch.randn(E, rows, cols, device="cuda")
+    m = torch.randn(E, rows, cols, device="cuda")
+    ms = m.clone()
+    u, ws = ns._prepare(m, g, 0.95, True, E)
+    for e in range(E):
+        u1, ws1 = ns._prepare(ms[e], g[e], 0.95, True, 1)
+        assert torch.equal(u[e], u1) and torch.equal(m[e], ms[e])
+        torch.testing.assert_close(ws[e, 0], ws1[0, 0], rtol=1e-5, atol=0)
+        torch.testing.assert_close(ws[e, 0], u1.float().square().sum(), rtol=1e-5, atol=0)
+    ops.check_status()
