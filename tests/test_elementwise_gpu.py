@@ -116,3 +116,27 @@ def test_cast_scale():
     c = torch.ones(5000, device=DEV)
     ew.cast_scale_(c, b, 2.0, accumulate=True)
     torch.testing.assert_close(c, 1 + 2 * b.float())
+
+
+@pytest.mark.parametrize("offset", [0, 4, 1])
+@pytest.mark.parametrize("gdt", [torch.float32, torch.bfloat16])
+def test_adamw_at_every_alignment(offset, gdt):
+    """32-byte, 16-byte and element-wise accesses give the same result, and it is that of fp64 arithmetic: moments to a few
+    fp32 roundings, a bf16 parameter to its own rounding (and, where that lies close to a tie, one step of it)."""
+    torch.manual_seed(12)
+    n = 8 * 1000 + 3
+    flat = lambda t: torch.cat([t.new_zeros(offset), t])[offset:]   # noqa: E731
+    p0 = torch.randn(n, device=DEV).bfloat16()
+    g0, m0 = torch.randn(n, device=DEV).to(gdt), torch.randn(n, device=DEV) * 0.1
+    v0 = torch.randn(n, device=DEV).square() * 10.0 ** torch.randint(-12, 1, (n,), device=DEV)
+    p, g, m, v = flat(p0), flat(g0), flat(m0), flat(v0)
+    ew.adamw_step_(p, g, m, v, lr=1e-2, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=3)
+    gd = g0.double()
+    md, vd = m0.double() * 0.9 + gd * 0.1, v0.double() * 0.95 + gd.square() * 0.05
+    step = 1e-2 / (1 - 0.9 ** 3) * md / (vd.sqrt() / (1 - 0.95 ** 3) ** 0.5 + 1e-8)
+    want = p0.double() * (1 - 1e-3) - step
+    mag = m0.abs().double() + gd.abs()
+    assert ((m.double() - md).abs() <= mag * 2.0 ** -22).all()
+    assert ((v.double() - vd).abs() <= vd * 2.0 ** -21).all()
+    assert ((p.double() - want).abs() <= (want.abs() * 2.0 ** -9 + (p0.abs().double() + step.abs()) * 2.0 ** -18)).all()
+    ops.check_status()
