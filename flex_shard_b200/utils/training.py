@@ -12,6 +12,8 @@ import time
 import torch
 import torch.distributed as dist
 
+from ..ops import multi_tensor
+
 
 def lr_lambda(step: int, warmup_steps: int, total_steps: int, decay_ratio: float = 0.0, min_lr_factor: float = 0.0):
     """Linear warm-up, constant plateau, linear decay over the last ``decay_ratio`` of training."""
@@ -25,34 +27,45 @@ def lr_lambda(step: int, warmup_steps: int, total_steps: int, decay_ratio: float
     return 1.0 - progress * (1.0 - min_lr_factor)
 
 
+def _native_grads(grads, norm_type, max_norm) -> bool:
+    """The multi-tensor kernels take the 2-norm of dense bf16 / fp32 gradients of one GPU."""
+    return (norm_type == 2 and isinstance(max_norm, (int, float))
+            and all(type(g) is torch.Tensor and g.is_cuda and g.device == grads[0].device and g.is_contiguous()
+                    and g.dtype in (torch.bfloat16, torch.float32) for g in grads))
+
+
 @torch.no_grad()
 def clip_grad_norm_(module, max_norm: float, norm_type: float = 2.0) -> torch.Tensor:
     """Global gradient norm over every bucket's local shards (one all-reduce per distinct mesh), then
-    scale the local gradients in place. Returns the total norm.  The per-parameter norms and the scaling run as
-    multi-tensor (``_foreach``) operations: a handful of launches instead of several per parameter."""
+    scale the local gradients in place. Returns the total norm.  The norms of a mesh's gradients are one pass over
+    all of them and so is the scaling (``csrc/grad_norm.cu``); gradients the kernels do not take (CPU, other norms or
+    dtypes) run as multi-tensor (``_foreach``) operations."""
     by_group: dict = {}
-    all_grads = []
     for st in module.sharded_bucket_storages:
         # every rank takes part in every mesh's all-reduce, with zero when it holds no gradient there (an owner
         # placement can leave a rank without any local rows)
-        acc = by_group.setdefault(id(st.comm.group), [st.comm, torch.zeros((), dtype=torch.float32, device=st.device)])
-        grads = [p.grad for p in st.sharded_params if p.grad is not None and p.grad.numel() > 0]
-        if not grads:
-            continue
-        all_grads += grads
-        norms = torch.stack(torch._foreach_norm(grads, norm_type, dtype=torch.float32))
-        acc[1] = acc[1] + (norms ** norm_type).sum()
+        acc = by_group.setdefault(id(st.comm.group), [st.comm, st.device, []])
+        acc[2] += [p.grad for p in st.sharded_params if p.grad is not None and p.grad.numel() > 0]
     total = None
-    for comm, v in by_group.values():
+    for comm, device, grads in by_group.values():
+        if not grads:
+            v = torch.zeros((), dtype=torch.float32, device=device)
+        elif _native_grads(grads, norm_type, max_norm):
+            v = multi_tensor.sum_squares(grads)
+        else:
+            norms = torch.stack(torch._foreach_norm(grads, norm_type, dtype=torch.float32))
+            v = (norms ** norm_type).sum()
         if comm.world_size > 1:
             dist.all_reduce(v, group=comm.group)
         total = v if total is None else total + v
     if total is None:
         return torch.zeros(())
     total_norm = total ** (1.0 / norm_type)
-    coef = (max_norm / (total_norm + 1e-6)).clamp(max=1.0)
-    if all_grads:
-        torch._foreach_mul_(all_grads, coef)
+    all_grads = [g for _, _, grads in by_group.values() for g in grads]
+    if all_grads and _native_grads(all_grads, norm_type, max_norm) and total_norm.device == all_grads[0].device:
+        multi_tensor.clip_by_norm_(all_grads, total_norm, max_norm)
+    elif all_grads:
+        torch._foreach_mul_(all_grads, (max_norm / (total_norm + 1e-6)).clamp(max=1.0))
     return total_norm
 
 

@@ -140,3 +140,30 @@ def test_adamw_at_every_alignment(offset, gdt):
     assert ((v.double() - vd).abs() <= vd * 2.0 ** -21).all()
     assert ((p.double() - want).abs() <= (want.abs() * 2.0 ** -9 + (p0.abs().double() + step.abs()) * 2.0 ** -18)).all()
     ops.check_status()
+
+
+@pytest.mark.parametrize("sizes", [[1], [7, 32768, 32769, 65543], [3] * 97 + [200001]])
+def test_clip_over_many_tensors(sizes):
+    """Edges: one element, a chunk and one more, odd remainders, unaligned views, more tensors than a launch takes."""
+    from flex_shard_b200.ops import multi_tensor
+
+    torch.manual_seed(11)
+    base = [torch.randn(n + 1, device=DEV) for n in sizes]
+    grads = [b[i % 2:i % 2 + n] if i % 3 else b[:n].bfloat16() for i, (b, n) in enumerate(zip(base, sizes))]
+    want = torch.stack([g.double().square().sum() for g in grads]).sum()
+    got = multi_tensor.sum_squares(grads)
+    # fp32 partial sums of at most 128 terms a thread and a tree over them: well within 200 roundings of 2^-24
+    assert abs(float(got) - float(want)) <= 1.2e-5 * float(want)
+    norm = got.sqrt()
+    limit = 0.25 * float(norm)
+    ref = [g.double() * (limit / (float(norm) + 1e-6)) for g in grads]
+    kept = [g.clone() for g in grads]
+    multi_tensor.clip_by_norm_(grads, norm, 2 * float(norm))            # below the limit: bit for bit the same
+    assert all(torch.equal(a, b) for a, b in zip(grads, kept))
+    multi_tensor.clip_by_norm_(grads, norm, limit)
+    for g, r in zip(grads, ref):
+        # one rounding of the product to the stored type, plus three fp32 roundings in the coefficient
+        torch.testing.assert_close(g.double(), r, rtol=2.0 ** -8 if g.dtype == torch.bfloat16 else 2.0 ** -21, atol=0)
+    multi_tensor.clip_by_norm_(grads, torch.full((), float("nan"), device=DEV), 1.0)
+    assert all(g.isnan().all() for g in grads)
+    ops.check_status()
