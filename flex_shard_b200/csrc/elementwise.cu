@@ -469,6 +469,25 @@ cross_entropy_resident_kernel(__nv_bfloat16* __restrict__ logits, const long lon
   }
 }
 
+// x[0, n) *= *scale in place, without touching x when the scale is 1. What a cross-entropy whose loss is not known to be
+// the root of backward() needs: the gradient of the loss is a device scalar that is 1 in nearly every program, and the
+// element-wise product into a new tensor moved 3.4 GB (1.88 ms) for 8192 x 102400 logits; reading the scalar takes 3 us.
+__global__ void __launch_bounds__(256)
+scale_by_scalar_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ scale, long long n) {
+  const float s = *scale;
+  if (s == 1.f) return;
+  const long long tid = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+  for (long long i = tid; i < n / 8; i += stride) {
+    float f[8];
+    load8(x + i * 8, f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] *= s;
+    store8(x + i * 8, f);
+  }
+  for (long long i = n / 8 * 8 + tid; i < n; i += stride) x[i] = __float2bfloat16(__bfloat162float(x[i]) * s);
+}
+
 // ------------------------------------------------------------------ AdamW over a flat shard
 // p: fp32 or bf16 master; g: fp32 or bf16; m, v: fp32. Optional `p_lowp`
 // receives the updated parameter as bf16 (the all-gather send buffer when the
@@ -824,6 +843,13 @@ FSB_API int fsb_segment_op_host(const void* host_descs, int nseg, int blocks_per
 }
 
 // step >= 1. p_fp32 / g_fp32 select the master and gradient dtypes.
+FSB_API int fsb_scale_by_scalar(void* x, const float* scale, long long n, cudaStream_t stream) {
+  if ((reinterpret_cast<uintptr_t>(x) & 15) != 0) return FSB_ERR_BAD_ARG;
+  if (n <= 0) return FSB_OK;
+  scale_by_scalar_kernel<<<grid_for(n, 256, 32), 256, 0, stream>>>(static_cast<__nv_bfloat16*>(x), scale, n);
+  return launch_ok();
+}
+
 FSB_API int fsb_adamw(void* p, const void* g, float* m, float* v, void* p_lowp, long long n,
                       int p_fp32, int g_fp32, float lr, float beta1, float beta2, float eps,
                       float weight_decay, int step, float grad_scale, cudaStream_t stream) {

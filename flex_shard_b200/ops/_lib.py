@@ -96,6 +96,7 @@ def _declare(lib) -> None:
         "fsb_swiglu_fwd": [vp, vp, i64, i32, vp],
         "fsb_swiglu_bwd": [vp, vp, vp, i64, i32, vp],
         "fsb_cross_entropy": [vp, vp, vp, i64, i32, i64, f32, i64, vp],
+        "fsb_scale_by_scalar": [vp, vp, i64, vp],
         "fsb_adamw": [vp, vp, vp, vp, vp, i64, i32, i32, f32, f32, f32, f32, f32, i32, f32, vp],
         "fsb_cast_scale": [vp, vp, i64, i32, f32, i32, vp],
         "fsb_segment_op": [vp, i32, i32, vp],

@@ -277,6 +277,15 @@ class _CrossEntropy(torch.autograd.Function):
         (dlogits,) = ctx.saved_tensors
         if ctx.unit_grad:
             return dlogits, None, None, None, None
+        if (dlogits.is_cuda and dlogits.is_contiguous() and dlogits.data_ptr() % 16 == 0 and dlogits.dtype == torch.bfloat16
+                and dloss.device == dlogits.device and dloss.dtype == torch.float32
+                and not torch._C._autograd._get_current_graph_task_keep_graph()):
+            # this graph is not run again, so its saved tensor can be scaled in place (a no-op when the gradient is 1)
+            rc = _lib.load().fsb_scale_by_scalar(dlogits.data_ptr(), dloss.data_ptr(), dlogits.numel(),
+                                                 _s(dlogits.device))
+            _lib.check(rc, "fsb_scale_by_scalar")
+            count_launch()
+            return dlogits, None, None, None, None
         return dlogits * dloss.to(dlogits.dtype), None, None, None, None
 
 

@@ -167,3 +167,24 @@ def test_clip_over_many_tensors(sizes):
     multi_tensor.clip_by_norm_(grads, torch.full((), float("nan"), device=DEV), 1.0)
     assert all(g.isnan().all() for g in grads)
     ops.check_status()
+
+
+@pytest.mark.parametrize("shape", [(3, 8), (5, 1000), (257, 4096)])
+@pytest.mark.parametrize("factor", [1.0, 0.37])
+def test_cross_entropy_gradient_of_a_scaled_loss(shape, factor):
+    """The saved gradient is scaled in place when the graph ends with this backward and kept when it does not."""
+    torch.manual_seed(3)
+    x = torch.randn(*shape, device=DEV).bfloat16()
+    target = torch.randint(0, shape[1], (shape[0],), device=DEV)
+    ref = x.double().requires_grad_()
+    (torch.nn.functional.cross_entropy(ref, target) * factor).backward()
+    leaf = x.clone().requires_grad_()
+    loss = ew.cross_entropy(leaf.clone(), target) * factor
+    again = torch.autograd.grad(loss, leaf, retain_graph=True)[0].clone()
+    twice = torch.autograd.grad(loss, leaf, retain_graph=True)[0].clone()
+    last = torch.autograd.grad(loss, leaf)[0]
+    for got in (again, twice, last):
+        # two roundings to bf16 (the saved gradient, its scaled copy) of values below 1 / T
+        torch.testing.assert_close(got.double(), ref.grad, rtol=2.0 ** -7, atol=2.0 ** -12 / shape[0])
+    assert torch.equal(again, twice)
+    ops.check_status()
