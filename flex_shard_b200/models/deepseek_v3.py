@@ -4,7 +4,8 @@ Hot ops run on this library's kernels: every projection is a tcgen05 GEMM, the r
 grouped tcgen05 GEMMs over an expert-major token layout planned on the device (no host sync),
 norms / SwiGLU / cross-entropy are the fused bandwidth kernels. Multi-head latent attention has
 192-wide query/key heads and 128-wide value heads; the flash-attention kernel of this library is
-specialised for 128/128, so MLA's softmax(QK^T)V itself runs on PyTorch's SDPA here.
+specialised for 128/128, so MLA's softmax(QK^T)V itself runs on PyTorch's SDPA here; its operands (rotary
+parts, the shared rotary key, the separated values) are laid out by one kernel each way (``ops/mla.py``).
 
 Role parity: ``examples/deepseek_v3/model.py`` of the reference (a plain-PyTorch DeepSeek-V3 with
 sigmoid top-k routing, an auxiliary-loss-free expert bias and shared experts); parameters are
@@ -21,6 +22,7 @@ import torch.nn.functional as F
 from ..ops import elementwise as ew
 from ..ops import moe as moe_ops
 from ..ops.gemm import linear
+from ..ops.mla import mla_operands
 
 
 @dataclass
@@ -86,12 +88,7 @@ class MLA(nn.Module):
         c_kv, k_pe = kv.split([cfg.kv_lora_rank, cfg.qk_rope_dim], dim=-1)
         kvb = linear(_rms(c_kv.contiguous(), self.kv_norm, cfg.norm_eps), self.wkv_b).view(
             B, S, H, cfg.qk_nope_dim + cfg.v_dim)
-        k_nope, v = kvb.split([cfg.qk_nope_dim, cfg.v_dim], dim=-1)
-        q_nope, q_pe = q.split([cfg.qk_nope_dim, cfg.qk_rope_dim], dim=-1)
-        q_pe = ew._rope_ref(q_pe, rope_table, False)
-        k_pe = ew._rope_ref(k_pe.reshape(B, S, 1, cfg.qk_rope_dim), rope_table, False)
-        qf = torch.cat([q_nope, q_pe], dim=-1)
-        kf = torch.cat([k_nope, k_pe.expand(B, S, H, cfg.qk_rope_dim)], dim=-1)
+        qf, kf, v = mla_operands(q, kvb, k_pe, rope_table, cfg.qk_nope_dim)
         # doc_mask [B, 1, S, S] (True = attend): causal within documents; without it plain causal attention
         o = F.scaled_dot_product_attention(qf.transpose(1, 2), kf.transpose(1, 2), v.transpose(1, 2),
                                            attn_mask=doc_mask, is_causal=doc_mask is None,

@@ -353,3 +353,29 @@ def test_shared_parameter_is_stored_once():
     assert len(list(m.parameters())) == 1
     m(torch.randint(0, 10, (3, 5))).square().mean().backward()
     assert m.emb.weight.grad is not None and m.out.weight is m.emb.weight
+
+
+@pytest.mark.parametrize("factor", [None, 1.0, 4.0])
+@pytest.mark.parametrize("storage,reduce", [(torch.bfloat16, torch.float32), (torch.float32, torch.float32),
+                                            (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
+def test_one_rank_reduction_equals_the_packed_one(storage, reduce, factor, monkeypatch):
+    """Gradients that skip the round trip through the reduce dtype on one rank are bit for bit those that take it, over
+    accumulated backwards and with a divisor; where the trip would round, it is taken."""
+    from flex_shard_b200 import BucketSpec, MixedPrecisionPolicy, flex_shard
+    from flex_shard_b200.placements.shard import Shard
+
+    res = []
+    for packed in (False, True):
+        if packed:
+            monkeypatch.setattr(Shard, "_reduces_to_itself", staticmethod(lambda *a: False))
+        torch.manual_seed(0)
+        m = Net().to(storage)
+        kw = {} if factor is None else dict(gradient_divide_factor=factor)
+        mp = MixedPrecisionPolicy(param_dtype=torch.bfloat16, reduce_dtype=reduce)
+        flex_shard(m, [BucketSpec(["a.*"], mp_policy=mp, **kw), BucketSpec(["b.*"], mp_policy=mp, **kw)])
+        for i in range(2):
+            x = torch.randn(5, 8, generator=torch.Generator().manual_seed(i)).bfloat16()
+            m(x).float().square().sum().backward()
+        res.append([p.grad for p in m.parameters()])
+    for a, b in zip(*res):
+        assert a.dtype == b.dtype == storage and torch.equal(a, b)

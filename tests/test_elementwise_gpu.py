@@ -118,7 +118,7 @@ def test_cast_scale():
     torch.testing.assert_close(c, 1 + 2 * b.float())
 
 
-@pytest.mark.parametrize("offset", [0, 4, 1])
+@pytest.mark.parametrize("offset", [0, 8, 1])
 @pytest.mark.parametrize("gdt", [torch.float32, torch.bfloat16])
 def test_adamw_at_every_alignment(offset, gdt):
     """32-byte, 16-byte and element-wise accesses give the same result, and it is that of fp64 arithmetic: moments to a few
@@ -138,7 +138,7 @@ def test_adamw_at_every_alignment(offset, gdt):
     mag = m0.abs().double() + gd.abs()
     assert ((m.double() - md).abs() <= mag * 2.0 ** -22).all()
     assert ((v.double() - vd).abs() <= vd * 2.0 ** -21).all()
-    assert ((p.double() - want).abs() <= (want.abs() * 2.0 ** -9 + (p0.abs().double() + step.abs()) * 2.0 ** -18)).all()
+    assert ((p.double() - want).abs() <= (want.abs() * 2.0 ** -8 + (p0.abs().double() + step.abs()) * 2.0 ** -18)).all()
     ops.check_status()
 
 

@@ -73,3 +73,30 @@ def test_route_plan_kernel_equals_operator_plan(T, k, E):
         assert torch.equal(got.tile_expert.cpu()[:n_tiles], want.tile_expert[:n_tiles])
         assert got.max_rows == want.max_rows
     ops.check_status()
+
+
+@pytest.mark.parametrize("B,S,H,nope,rope,value", [(1, 1, 1, 8, 8, 8), (2, 37, 3, 64, 32, 64), (1, 200, 16, 128, 64, 128),
+                                                   (3, 5, 5, 24, 16, 40)])
+def test_latent_attention_operands_match_the_torch_steps(B, S, H, nope, rope, value):
+    from flex_shard_b200.ops import elementwise as ew
+    from flex_shard_b200.ops import mla
+
+    torch.manual_seed(8)
+    dev = torch.device("cuda")
+    table = ew.rope_table(S + 3, rope, 10000.0, dev)[:S]
+    q = torch.randn(B, S, H, nope + rope, device=dev).bfloat16()
+    kvb = torch.randn(B, S, H, nope + value, device=dev).bfloat16()
+    kv = torch.randn(B, S, 16 + rope, device=dev).bfloat16()
+    grads = [torch.randn(B, S, H, n, device=dev).bfloat16() for n in (nope + rope, nope + rope, value)]
+    grads[0] = grads[0].transpose(1, 2).contiguous().transpose(1, 2)     # another memory order than the outputs'
+    assert mla._native(q, kvb, kv[..., 16:], table, nope)
+    res = []
+    for fn, cast in ((mla.mla_operands, lambda t: t), (mla.mla_operands_ref, torch.Tensor.double)):
+        leaves = [cast(t).clone().requires_grad_() for t in (q, kvb, kv)]
+        outs = fn(leaves[0], leaves[1], leaves[2][..., 16:], table, nope)
+        torch.autograd.backward(outs, [cast(g) for g in grads])
+        res.append([t.detach().double() for t in (*outs, *(x.grad for x in leaves))])
+    for got, ref in zip(*res):
+        # the reference rotates in fp32 (2^-22 of |x| + |y| < 2^3 H) on double inputs; one rounding to bf16 on top
+        assert ((got - ref).abs() <= ref.abs() * 2.0 ** -8 + H * 2.0 ** -18).all()
+    ops.check_status()
