@@ -102,3 +102,29 @@ def test_weight_gradient_product_reads_both_operands_transposed(T, N, K):
     ops.check_status()
     ref = mx.gemm_mxfp8(dq.cpu(), sd.cpu(), xq.cpu(), sx.cpu(), a_t=True, b_t=True, out_dtype=torch.float32)
     torch.testing.assert_close(dw.cpu(), ref, rtol=1e-3, atol=1e-3 * T ** 0.5)
+
+
+@pytest.mark.parametrize("M,N,K,a_t,b_t,dt", [
+    (2432, 2432, 256, False, False, torch.float32), (2305, 2440, 128, False, False, torch.bfloat16),
+    (4104, 1560, 384, False, False, torch.float32), (2320, 2448, 256, False, True, torch.bfloat16),
+    (2448, 2320, 640, True, True, torch.float32), (2432, 4112, 128, True, False, torch.bfloat16)])
+def test_block_scaled_gemm_on_sm_pairs(M, N, K, a_t, b_t, dt):
+    """Outputs of more than one wave of 128 x 128 tiles run on SM pairs: half tiles, ragged edges, every operand major.
+    Products of 8-bit values and powers of two are exact, sums of K of them good to K 2^-24 of the sum of magnitudes."""
+    g = torch.Generator().manual_seed(7)
+    dev = torch.device("cuda")
+
+    def operand(rows):
+        q, s = mx.mx_quantize_act_ref((torch.randn(rows, K, generator=g) * torch.rand(rows, 1, generator=g)).bfloat16())
+        e = mx.from_blocked(s, rows, K // 32)
+        return q, s, q.double() * torch.exp2(e.double() - 127).repeat_interleave(32, 1)
+
+    aq, sa, a = operand(M)
+    bq, sb, b = operand(N)
+    dq = lambda q, t: (q.view(torch.uint8).t().contiguous().view(q.dtype) if t else q).to(dev)   # noqa: E731
+    y = mx.gemm_mxfp8(dq(aq, a_t), sa.to(dev), dq(bq, b_t), sb.to(dev), a_t=a_t, b_t=b_t, out_dtype=dt)
+    ops.check_status()
+    a, b = a.to(dev), b.to(dev)
+    ref = a @ b.t()
+    bound = (a.abs() @ b.abs().t()) * (K * 2.0 ** -24) + ref.abs() * (2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -23)
+    assert ((y.double() - ref).abs() <= bound).all()
