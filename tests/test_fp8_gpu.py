@@ -100,3 +100,12 @@ def test_stacked_fp8_linear_runs_every_matrix_through_its_own_tiles():
     assert (y.float() - yr).abs().max() < 0.15 * yr.abs().max()
     assert (x.grad.float() - xr.grad).abs().max() < 0.15 * xr.grad.abs().max()
     torch.testing.assert_close(lin.weight.grad.float(), wr.grad, rtol=3e-2, atol=3e-1)
+
+
+@pytest.mark.parametrize("T,K,pad", [(1, 128, 0), (33, 384, 4), (130, 256, 12), (257, 2048, 16)])
+def test_act_quantiser_on_strided_inputs(T, K, pad):
+    torch.manual_seed(7)
+    x = torch.randn(T, K + pad, device=DEV).bfloat16()[:, pad:]
+    q, s = fp8.quantize_act(x)
+    qr, sr = fp8.quantize_act_ref(x.contiguous())
+    assert torch.equal(q.view(torch.uint8), qr.view(torch.uint8)) and torch.equal(s, sr)

@@ -128,3 +128,25 @@ def test_block_scaled_gemm_on_sm_pairs(M, N, K, a_t, b_t, dt):
     ref = a @ b.t()
     bound = (a.abs() @ b.abs().t()) * (K * 2.0 ** -24) + ref.abs() * (2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -23)
     assert ((y.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("rows,cols,pad", [(33, 40, 0), (64, 130, 6), (31, 96, 3), (128, 128, 1), (256, 384, 8)])
+def test_quantisers_on_strided_and_unaligned_inputs(rows, cols, pad):
+    """Row strides off the 16-byte grid, columns that end inside a tile, tiles that end inside a block."""
+    torch.manual_seed(9)
+    base = (torch.randn(rows, cols + pad) * 3).bfloat16()
+    q_ref, e_ref = mx.mx_quantize_weight(base[:, pad:])
+    q, e = mx.mx_quantize_weight(base.cuda()[:, pad:])
+    assert torch.equal(e.cpu(), e_ref) and torch.equal(q.cpu().view(torch.uint8), q_ref.view(torch.uint8))
+    pad = pad // 4 * 4                                          # activations: 4-element granularity of the row stride
+    wide = (torch.randn(rows, 384 + pad) * 3).bfloat16()
+    q_ref, s_ref = mx.mx_quantize_act(wide[:, pad:])
+    q, s = mx.mx_quantize_act(wide.cuda()[:, pad:])
+    assert torch.equal(q.cpu().view(torch.uint8), q_ref.view(torch.uint8))
+    assert torch.equal(mx.from_blocked(s.cpu(), rows, 12), mx.from_blocked(s_ref, rows, 12))
+    if rows % 128 == 0:
+        for p in (pad, 1):
+            wide = (torch.randn(rows, 384 + p) * 3).bfloat16()
+            q_ref, s_ref = mx.mx_quantize_rows(wide[:, p:])
+            q, s = mx.mx_quantize_rows(wide.cuda()[:, p:])
+            assert torch.equal(q.cpu().view(torch.uint8), q_ref.view(torch.uint8)) and torch.equal(s.cpu(), s_ref)
