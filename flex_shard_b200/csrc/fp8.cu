@@ -128,11 +128,17 @@ quant_act_1x128_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict_
 
 // ------------------------------------------------------------------ block-scaled GEMM
 constexpr int BM = 128, BN = 128, BK = 128;  // BK bytes == elements (fp8)
-constexpr int STAGES = 5;
+constexpr int STAGES = 6;
+constexpr int BUFS = 4;                      // block products in TMEM: 4 x 128 columns
 constexpr int A_STAGE = BM * BK, B_STAGE = BN * BK, STAGE_BYTES = A_STAGE + B_STAGE;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
 constexpr int NUM_THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2..9 scale-accumulate (two per lane quarter)
 
+// Every 128-deep block is a product of its own, whose 128 x 128 fp32 values leave TMEM and are folded into registers with
+// the block's scales: bound by that chain (wait, TMEM read, FMA) per block and warp, not by a unit (ncu, when it read and
+// folded in turn from two buffers: tensor pipe 31 %, L2 37 %, issue slots 35 %). So the read of the next 32 columns, or
+// of the next block, is in flight while 32 columns are folded with two-element FMAs, and four buffers keep the tensor core
+// ahead.
 struct Fp8Args {
   int M, N, K;
   int b_mn;
@@ -144,6 +150,11 @@ struct Fp8Args {
   int* status;
 };
 
+// acc (two fp32) = v * s + acc, one instruction for both
+__device__ __forceinline__ void fma2(unsigned long long& acc, uint32_t v0, uint32_t v1, unsigned long long s2) {
+  asm("{\n\t.reg .b64 v;\n\tmov.b64 v, {%1, %2};\n\tfma.rn.f32x2 %0, v, %3, %0;\n\t}" : "+l"(acc) : "r"(v0), "r"(v1), "l"(s2));
+}
+
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                 const Fp8Args args) {
@@ -153,9 +164,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + STAGES;
-  uint64_t* tmem_full = bars + 2 * STAGES;       // [2]
-  uint64_t* tmem_empty = bars + 2 * STAGES + 2;  // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+  uint64_t* tmem_full = bars + 2 * STAGES;          // [BUFS]
+  uint64_t* tmem_empty = bars + 2 * STAGES + BUFS;  // [BUFS]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2 * BUFS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -168,7 +179,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < BUFS; ++i) {
       mbar_init(&tmem_full[i], 1);
       mbar_init(&tmem_empty[i], 8);
     }
@@ -176,7 +187,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     mbar_fence_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 256);
+    tmem_alloc(tmem_slot, BUFS * BN);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -191,7 +202,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       uint32_t it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const int tm = tile % tiles_m, tn = tile / tiles_m;
+        int tm, tn;
+        grouped_tile_coords(tile, tiles_m, tiles_n, tm, tn);
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -225,7 +237,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         for (int kb = 0; kb < num_kb; ++kb, ++it, ++blk) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
-          const uint32_t buf = blk & 1, bph = (blk >> 1) & 1;
+          const uint32_t buf = blk % BUFS, bph = (blk / BUFS) & 1;
           if (!mbar_wait(&full_bar[s], ph, abort_flag) || !mbar_wait(&tmem_empty[buf], bph ^ 1, abort_flag)) {
             if (lane == 0) {
               atomicExch(args.status, FSB_ERR_WAIT_TIMEOUT_FULL);
@@ -254,45 +266,68 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const int quarter = warp & 3;
     const int half = (warp - 2) >> 2;
     constexpr int HC = BN / 2;
-    const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * HC;
     uint32_t blk = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-      const int tm = tile % tiles_m, tn = tile / tiles_m;
-      const long long row = static_cast<long long>(tm) * BM + quarter * 32 + lane;
-      const bool row_ok = row < args.M;
-      float acc[HC];
-#pragma unroll
-      for (int i = 0; i < HC; ++i) acc[i] = 0.f;
-      for (int kb = 0; kb < num_kb; ++kb, ++blk) {
-        const uint32_t buf = blk & 1, bph = (blk >> 1) & 1;
-        const float s = (row_ok ? args.sa[static_cast<long long>(kb) * args.M + row] : 0.f) *
-                        args.sb[tn * args.sb_stride_n + kb * args.sb_stride_k];
-        if (!mbar_wait(&tmem_full[buf], bph, abort_flag)) {
-          if (lane == 0) {
-            atomicExch(args.status, FSB_ERR_WAIT_TIMEOUT_TMEM_FULL);
-            *abort_flag = 1;
-          }
-          ok = false;
-          break;
-        }
+    auto wait_full = [&](uint32_t b) {
+      if (mbar_wait_warp(&tmem_full[b % BUFS], (b / BUFS) & 1, abort_flag)) {
         tc_fence_after();
-        uint32_t v0[32], v1[32];
-        tmem_ld_32x32(tmem_base + lane_off + buf * BN + half * HC, v0);
-        tmem_ld_32x32(tmem_base + lane_off + buf * BN + half * HC + 32, v1);
-        tmem_ld_wait();
+        return true;
+      }
+      if (lane == 0) {
+        atomicExch(args.status, FSB_ERR_WAIT_TIMEOUT_TMEM_FULL);
+        *abort_flag = 1;
+      }
+      return false;
+    };
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      int tm, tn;
+      grouped_tile_coords(tile, tiles_m, tiles_n, tm, tn);
+      const int row = tm * BM + quarter * 32 + lane;
+      const bool row_ok = row < args.M;
+      unsigned long long acc2[HC / 2];
+#pragma unroll
+      for (int i = 0; i < HC / 2; ++i) acc2[i] = 0ull;
+      // the scales of a block are loaded one block ahead: their latency is longer than a block
+      const float* pa = args.sa + (row_ok ? row : 0);
+      const float* pb = args.sb + tn * args.sb_stride_n;
+      float next_a = row_ok ? *pa : 0.f, next_b = *pb;
+      uint32_t v0[32], v1[32];
+      ok = wait_full(blk);
+      if (ok) tmem_ld_32x32(t_row + (blk % BUFS) * BN, v0);
+      for (int kb = 0; kb < num_kb && ok; ++kb, ++blk) {
+        const uint32_t buf = blk % BUFS;
+        const float s = next_a * next_b;
+        if (kb + 1 < num_kb) {
+          pa += args.M;
+          pb += args.sb_stride_k;
+          next_a = row_ok ? *pa : 0.f;
+          next_b = *pb;
+        }
+        unsigned long long s2;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(s2) : "f"(s));
+        tmem_ld_wait_for(v0);
+        tmem_ld_32x32(t_row + buf * BN + 32, v1);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) fma2(acc2[i], v0[2 * i], v0[2 * i + 1], s2);
+        tmem_ld_wait_for(v1);
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&tmem_empty[buf]);  // values are in registers: free the buffer early
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          acc[i] = fmaf(s, __uint_as_float(v0[i]), acc[i]);
-          acc[32 + i] = fmaf(s, __uint_as_float(v1[i]), acc[32 + i]);
+        if (lane == 0) mbar_arrive(&tmem_empty[buf]);  // the block is in registers
+        if (kb + 1 < num_kb) {
+          ok = wait_full(blk + 1);
+          if (ok) tmem_ld_32x32(t_row + ((blk + 1) % BUFS) * BN, v0);
         }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) fma2(acc2[16 + i], v1[2 * i], v1[2 * i + 1], s2);
       }
+      if (!ok) tmem_ld_wait();   // nothing may be in flight when TMEM is given back
+      float acc[HC];
+#pragma unroll
+      for (int i = 0; i < HC / 2; ++i) asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[2 * i]), "=f"(acc[2 * i + 1]) : "l"(acc2[i]));
       if (ok && row_ok) {
         const int cbase = tn * BN + half * HC;
-        __nv_bfloat16* dp = args.d + row * args.ldd + cbase;
+        __nv_bfloat16* dp = args.d + static_cast<long long>(row) * args.ldd + cbase;
         const int ncols = min(HC, args.N - cbase);
         if (ncols == HC && (args.ldd % 8) == 0) {
 #pragma unroll
@@ -322,7 +357,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       }
     }
     tc_fence_after();
-    tmem_dealloc(tmem_base, 256);
+    tmem_dealloc(tmem_base, BUFS * BN);
   }
 }
 

@@ -102,6 +102,40 @@ def test_stacked_fp8_linear_runs_every_matrix_through_its_own_tiles():
     torch.testing.assert_close(lin.weight.grad.float(), wr.grad, rtol=3e-2, atol=3e-1)
 
 
+@pytest.mark.parametrize("M,N,K", [(2432, 2432, 256), (2305, 2448, 128), (4104, 1552, 384), (128, 19200, 256)])
+def test_fp8_gemm_at_ragged_sizes(M, N, K):
+    """More than one tile per SM, ragged rows and columns, one block of depth (fewer than the buffers between the tensor
+    core and the folding warps), a single row tile. Products of 8-bit values are exact in fp32, sums of K of them are good to K 2^-24 of the sum
+    of magnitudes, and the result is rounded to bf16 once."""
+    torch.manual_seed(5)
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    w = torch.randn(N, K, device=DEV).bfloat16()
+    wq, ws = fp8.quantize_blockwise(w)
+    xq, sx = fp8.quantize_act(x)
+    a = (xq.double().view(M, K // 128, 128) * sx.double().t()[..., None]).view(M, K)
+    b = wq.double() * ws.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)
+    got = fp8.gemm_fp8(xq, sx, wq, ws)
+    ops.check_status()
+    bound = (a.abs() @ b.t().abs()) * (K * 2.0 ** -24)
+    ref = a @ b.t()
+    assert ((got.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + bound).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(2432, 256, 2432), (2304, 128, 2320), (4104, 384, 1552)])
+def test_fp8_gemm_transposed_at_ragged_sizes(M, N, K):
+    """Input gradients: the weight [N, K] is read as its transpose, so the output is [M, K]."""
+    torch.manual_seed(6)
+    wq, ws = fp8.quantize_blockwise(torch.randn(N, K, device=DEV).bfloat16())
+    dq, sd = fp8.quantize_act(torch.randn(M, N, device=DEV).bfloat16())
+    a = (dq.double().view(M, N // 128, 128) * sd.double().t()[..., None]).view(M, N)
+    b = wq.double() * ws.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)[:, :K]
+    got = fp8.gemm_fp8(dq, sd, wq, ws, b_t=True)
+    ops.check_status()
+    ref = a @ b
+    bound = (a.abs() @ b.abs()) * (N * 2.0 ** -24)
+    assert ((got.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + bound).all()
+
+
 @pytest.mark.parametrize("T,K,pad", [(1, 128, 0), (33, 384, 4), (130, 256, 12), (257, 2048, 16)])
 def test_act_quantiser_on_strided_inputs(T, K, pad):
     torch.manual_seed(7)
