@@ -657,11 +657,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // tcgen05.commit arrives on the `empty` / `tmem_full` barriers of both CTAs; the epilogue warps of
 // both CTAs arrive on CTA 0's `tmem_empty` barrier. Every wait is bounded; a CTA that gives up
 // still walks to the cluster barrier at the end, so its peer is never left alone.
+constexpr int kDense = 0, kBatched = 1, kGrouped = 2;   // forms of the two-SM kernel
 constexpr int BN_HALF = 128;                       // B rows per CTA
 constexpr int STAGES2 = 6;
 constexpr int B2_STAGE_BYTES = BN_HALF * BK * 2;   // 16 KB
 constexpr int STAGE2_BYTES = A_STAGE_BYTES + B2_STAGE_BYTES;
 constexpr int SMEM2_BYTES = STAGES2 * STAGE2_BYTES + 1024 + 256 + EPI_STAGE_BYTES;
+constexpr int MAX_GROUPS2 = 256;                   // groups of the grouped form (its tables sit behind the staging tiles)
+constexpr int SMEM2_GROUPED_BYTES = SMEM2_BYTES + 2 * (MAX_GROUPS2 + 1) * 4;
 
 __device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr,
                                                  int32_t c0, int32_t c1, int32_t c2) {
@@ -671,10 +674,10 @@ __device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorM
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
-template <bool BATCH>
+template <int KIND>
 __device__ __forceinline__ void load_tile_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr,
                                                int32_t c0, int32_t c1, int32_t e) {
-  if constexpr (BATCH) tma_load_3d_pair(smem_dst, map, bar_cluster_addr, c0, c1, e);
+  if constexpr (KIND == kBatched) tma_load_3d_pair(smem_dst, map, bar_cluster_addr, c0, c1, e);
   else tma_load_2d_pair(smem_dst, map, bar_cluster_addr, c0, c1);
 }
 __device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
@@ -706,31 +709,65 @@ __device__ __forceinline__ void upper_tile_coords(int t, int T, int& tm, int& tn
 
 // Which 256x256 tile of which matrix a pair works on.
 struct PairTile {
-  int tm2, tn, e;
+  int tm, tn, e;        // 128-row tile of the pair's first CTA, 256-column tile, matrix or group
+  int num_kb, k0;       // 64-deep blocks and the first index of the contraction
+  int b_row;            // first row of the group's slice of B
+  int rows_end;         // rows of D from here on belong to the next group (or do not exist)
+  bool diagonal;
 };
-template <bool BATCH>
+template <int KIND>
 __device__ __forceinline__ PairTile pair_tile(const GemmArgs& args, int tile, int tiles_m, int tiles_n, int per_matrix,
-                                              bool spread) {
+                                              bool spread, const int* off, const int* first) {
   PairTile t;
   t.e = 0;
-  if (BATCH) {
+  t.num_kb = (args.K + BK - 1) / BK;
+  t.k0 = 0;
+  t.b_row = 0;
+  t.rows_end = args.M;
+  t.diagonal = true;
+  if (KIND == kGrouped && args.group_mode == 1) {
+    int lo = 0, hi = args.num_groups - 1;   // last group whose first tile is <= tile (empty groups own none)
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (first[mid] * tiles_n <= tile) lo = mid; else hi = mid - 1;
+    }
+    const int rows = first[lo + 1] - first[lo], local = tile - first[lo] * tiles_n;
+    t.e = lo;
+    t.tm = off[lo] / BM + 2 * (local % rows);
+    t.tn = local / rows;
+    t.b_row = lo * static_cast<int>(args.b_group_rows);
+    t.rows_end = off[lo + 1];
+    return t;
+  }
+  if (KIND != kDense) {
     t.e = tile / per_matrix;
     tile -= t.e * per_matrix;
   }
+  int tm2;
   if (args.upper_only) {
-    upper_tile_coords(tile, tiles_m, t.tm2, t.tn);
+    upper_tile_coords(tile, tiles_m, tm2, t.tn);
+    t.diagonal = tm2 == t.tn;
   } else {
-    tile_coords(tile, tiles_m, tiles_n, t.tm2, t.tn);
-    if (spread) t.tm2 = spread_over_row_blocks(t.tm2, tiles_m, args.d_peer_n);
+    tile_coords(tile, tiles_m, tiles_n, tm2, t.tn);
+    if (spread) tm2 = spread_over_row_blocks(tm2, tiles_m, args.d_peer_n);
+  }
+  t.tm = 2 * tm2;
+  if (KIND == kGrouped) {
+    t.k0 = off[t.e];
+    t.num_kb = (off[t.e + 1] - off[t.e]) / BK;
   }
   return t;
 }
 
-// BATCH: args.batch equal matrices per operand, addressed through 3-D tensor maps, so the edge of every matrix is
+// kBatched: args.batch equal matrices per operand, addressed through 3-D tensor maps, so the edge of every matrix is
 // filled with zeros and M, N, K need not be multiples of a tile. All matrices share one persistent grid: a stack of
 // small products (attention heads, experts) fills the SMs that a launch per matrix would leave idle, and each product
 // of a stack costs one launch.
-template <bool BATCH>
+// kGrouped: the grouped modes of GemmArgs on pairs. Row groups start on multiples of 128, so in mode 1 a group's last
+// tile may have only its first CTA's 128 rows: the second CTA then multiplies rows of the next group and stores nothing
+// (an eighth of the work at 768 rows a group, against twice the operand reads of a 128-row tile per SM). Every CTA
+// derives the tiles of the groups from the offsets in device memory.
+template <int KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                      const GemmArgs args) {
@@ -751,13 +788,33 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   const int tiles_m = (args.M + 2 * BM - 1) / (2 * BM);   // 256-row tiles
   const int tiles_n = (args.N + BN - 1) / BN;
   const int per_matrix = args.upper_only ? tiles_m * (tiles_m + 1) / 2 : tiles_m * tiles_n;
-  const int num_tiles = BATCH ? per_matrix * args.batch : per_matrix;
-  const int num_kb = (args.K + BK - 1) / BK;
+  int num_tiles = KIND == kBatched ? per_matrix * args.batch : KIND == kGrouped ? per_matrix * args.num_groups : per_matrix;
   const int tile0 = static_cast<int>(blockIdx.x >> 1);
   const int tile_step = static_cast<int>(gridDim.x >> 1);
   const bool spread = args.d_peer_remote && args.d_peer_n > 1 && args.d_block_rows % (2 * BM) == 0 &&
                       static_cast<long long>(tiles_m) * (2 * BM) == args.d_block_rows * args.d_peer_n;
+  int* off = reinterpret_cast<int*>(smem + STAGES2 * STAGE2_BYTES + 256 + EPI_STAGE_BYTES);   // [groups + 1] row offsets
+  int* first = off + MAX_GROUPS2 + 1;                                                         // [groups + 1] first row tile
 
+  if (KIND == kGrouped && warp == 2) {
+    int base = 0;
+    for (int g = 0; g <= args.num_groups; g += 32) {
+      const int i = g + lane;
+      const int o = i <= args.num_groups ? args.group_offs[i] : 0;
+      const int n = i < args.num_groups ? (args.group_offs[i + 1] - o + 2 * BM - 1) / (2 * BM) : 0;
+      int sum = n;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, sum, d);
+        if (lane >= d) sum += up;
+      }
+      if (i <= args.num_groups) {
+        off[i] = o;
+        first[i] = base + sum - n;
+      }
+      base += __shfl_sync(0xffffffffu, sum, 31);
+    }
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES2; ++s) {
       mbar_init(&full_bar[s], 1);
@@ -781,6 +838,7 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   cluster_sync_all();   // the peer's barriers are initialised before anything is signalled across the pair
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (KIND == kGrouped && args.group_mode == 1) num_tiles = first[args.num_groups] * tiles_n;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -790,10 +848,10 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       uint32_t it = 0;
       bool ok = true;
       for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
-        const PairTile pt = pair_tile<BATCH>(args, tile, tiles_m, tiles_n, per_matrix, spread);
-        const int m0 = pt.tm2 * 2 * BM + static_cast<int>(rank) * BM;
+        const PairTile pt = pair_tile<KIND>(args, tile, tiles_m, tiles_n, per_matrix, spread, off, first);
+        const int m0 = (pt.tm + static_cast<int>(rank)) * BM;
         const int n0 = pt.tn * BN + static_cast<int>(rank) * BN_HALF;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+        for (int kb = 0; kb < pt.num_kb; ++kb, ++it) {
           const int s = it % STAGES2;
           const uint32_t ph = (it / STAGES2) & 1;
           if (!mbar_wait(&empty_bar[s], ph ^ 1, abort_flag)) {
@@ -806,19 +864,19 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
           uint8_t* sb = sa + A_STAGE_BYTES;
           const uint32_t full0 = map_to_cta(smem_u32(&full_bar[s]), 0);
           if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * STAGE2_BYTES);   // the bytes of both CTAs
-          const int k0 = kb * BK;
+          const int k0 = pt.k0 + kb * BK;
           if (!args.a_mn) {
-            load_tile_pair<BATCH>(sa, &map_a, full0, k0, m0, pt.e);
+            load_tile_pair<KIND>(sa, &map_a, full0, k0, m0, pt.e);
           } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j) load_tile_pair<BATCH>(sa + j * 8192, &map_a, full0, m0 + 64 * j, k0, pt.e);
+            for (int j = 0; j < BM / 64; ++j) load_tile_pair<KIND>(sa + j * 8192, &map_a, full0, m0 + 64 * j, k0, pt.e);
           }
           if (!args.b_mn) {
-            load_tile_pair<BATCH>(sb, &map_b, full0, k0, n0, pt.e);
+            load_tile_pair<KIND>(sb, &map_b, full0, k0, pt.b_row + n0, pt.e);
           } else {
 #pragma unroll
             for (int j = 0; j < BN_HALF / 64; ++j)
-              load_tile_pair<BATCH>(sb + j * 8192, &map_b, full0, n0 + 64 * j, k0, pt.e);
+              load_tile_pair<KIND>(sb + j * 8192, &map_b, full0, n0 + 64 * j, pt.b_row + k0, pt.e);
           }
         }
       }
@@ -832,6 +890,9 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       uint32_t it = 0, local_tile = 0;
       bool ok = true;
       for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
+        const int num_kb = KIND == kGrouped ? pair_tile<KIND>(args, tile, tiles_m, tiles_n, per_matrix, spread, off, first).num_kb
+                                            : (args.K + BK - 1) / BK;
+        if (KIND == kGrouped && num_kb == 0) continue;
         const uint32_t acc = local_tile & 1;
         const uint32_t acc_ph = (local_tile >> 1) & 1;
         ++local_tile;
@@ -885,8 +946,21 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const int quarter = warp & 3;
     uint32_t local_tile = 0;
     for (int tile = tile0; tile < num_tiles; tile += tile_step) {
-      const PairTile pt = pair_tile<BATCH>(args, tile, tiles_m, tiles_n, per_matrix, spread);
-      const int tm = pt.tm2 * 2 + static_cast<int>(rank);
+      const PairTile pt = pair_tile<KIND>(args, tile, tiles_m, tiles_n, per_matrix, spread, off, first);
+      const int tm = pt.tm + static_cast<int>(rank);
+      const long long d_row_off = KIND == kBatched || (KIND == kGrouped && args.group_mode == 2) ? static_cast<long long>(pt.e) * args.M : 0;
+      if (KIND == kGrouped && pt.num_kb == 0) {
+        // an empty group contributes nothing: its output tile is zero (or left alone when accumulating)
+        const int row = tm * BM + quarter * 32 + lane;
+        if (row < args.M && !args.accumulate) {
+          for (int c = pt.tn * BN; c < min(args.N, pt.tn * BN + BN); ++c) {
+            const long long o = (d_row_off + row) * args.ldd + c;
+            if (args.d_fp32) static_cast<float*>(args.d)[o] = 0.f;
+            else static_cast<__nv_bfloat16*>(args.d)[o] = __float2bfloat16(0.f);
+          }
+        }
+        continue;
+      }
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_ph = (local_tile >> 1) & 1;
       ++local_tile;
@@ -898,10 +972,10 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         break;
       }
       tc_fence_after();
-      store_tile(args, BATCH ? static_cast<long long>(pt.e) * args.M : 0, tm, pt.tn,
+      if (KIND != kGrouped || tm * BM < pt.rows_end) store_tile(args, d_row_off, tm, pt.tn,
                  tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16),
                  reinterpret_cast<float*>(smem + STAGES2 * STAGE2_BYTES + 256) + (warp - 2) * 32 * 33, quarter, lane,
-                 args.upper_only && pt.tm2 != pt.tn);
+                 args.upper_only && !pt.diagonal);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
@@ -1032,10 +1106,12 @@ static inline bool g_use_pairs_fwd() { return g_use_pairs_value() != 0; }
 static int pair_clusters(int dev) {
   if (g_pair_clusters[dev] == 0) {
     int found = -1;
-    if (cudaFuncSetAttribute(gemm_bf16_2sm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES) ==
+    if (cudaFuncSetAttribute(gemm_bf16_2sm_kernel<kDense>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES) ==
             cudaSuccess &&
-        cudaFuncSetAttribute(gemm_bf16_2sm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES) ==
-            cudaSuccess) {
+        cudaFuncSetAttribute(gemm_bf16_2sm_kernel<kBatched>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES) ==
+            cudaSuccess &&
+        cudaFuncSetAttribute(gemm_bf16_2sm_kernel<kGrouped>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             SMEM2_GROUPED_BYTES) == cudaSuccess) {
       cudaLaunchConfig_t cfg{};
       cfg.gridDim = dim3(2, 1, 1);
       cfg.blockDim = dim3(NUM_THREADS, 1, 1);
@@ -1048,7 +1124,7 @@ static int pair_clusters(int dev) {
       cfg.attrs = &at;
       cfg.numAttrs = 1;
       int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, gemm_bf16_2sm_kernel<false>, &cfg) == cudaSuccess && n > 0) found = n;
+      if (cudaOccupancyMaxActiveClusters(&n, gemm_bf16_2sm_kernel<kDense>, &cfg) == cudaSuccess && n > 0) found = n;
     }
     cudaGetLastError();
     g_pair_clusters[dev] = found;
@@ -1092,7 +1168,7 @@ static int gemm_pair_launch(const void* a, const void* b, void* d, const void* c
     args.upper_only = 1;
   }
   const int clusters = tiles < g_pair_clusters[dev] ? static_cast<int>(tiles) : g_pair_clusters[dev];
-  gemm_bf16_2sm_kernel<false><<<2 * clusters, NUM_THREADS, SMEM2_BYTES, stream>>>(map_a, map_b, args);
+  gemm_bf16_2sm_kernel<kDense><<<2 * clusters, NUM_THREADS, SMEM2_BYTES, stream>>>(map_a, map_b, args);
   return cudaGetLastError() == cudaSuccess ? FSB_OK : FSB_ERR_LAUNCH;
 }
 
@@ -1131,7 +1207,7 @@ FSB_API int fsb_gemm_bf16_batched(const void* a, const void* b, void* d, const v
   args.upper_only = upper;
   args.status = status;
   const int clusters = tiles < g_pair_clusters[dev] ? static_cast<int>(tiles) : g_pair_clusters[dev];
-  gemm_bf16_2sm_kernel<true><<<2 * clusters, NUM_THREADS, SMEM2_BYTES, stream>>>(map_a, map_b, args);
+  gemm_bf16_2sm_kernel<kBatched><<<2 * clusters, NUM_THREADS, SMEM2_BYTES, stream>>>(map_a, map_b, args);
   return cudaGetLastError() == cudaSuccess ? FSB_OK : FSB_ERR_LAUNCH;
 }
 
@@ -1161,12 +1237,20 @@ FSB_API int fsb_gemm_bf16_grouped(const void* a, const void* b, void* d, int mod
   CUtensorMap map_a, map_b;
   int rc;
   GemmArgs args{};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return FSB_ERR_BAD_ARG;
+  // SM pairs where their 256 x 256 tiles are mostly full: row groups of two 128-row tiles or more on average, outputs of
+  // at least one tile per group. Eight products of 64 experts (49152 rows, 2816 x 2048 and 2048 x 1408): 3.16 ms on single
+  // SMs, 2.84 on pairs.
+  const bool pairs = g_use_pairs_fwd() && num_groups <= MAX_GROUPS2 && N >= BN && pair_clusters(dev) > 0 &&
+                     (mode == 1 ? max_rows >= 3ll * BM * num_groups : M >= 2 * BM);
   if (mode == 1) {
     // A [max_rows, K] K-major; B stacked over experts
     rc = fsb_make_tmap_2d(&map_a, a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, max_rows, K, lda, BM, BK);
     if (rc != FSB_OK) return rc;
     if (!b_mn) rc = fsb_make_tmap_2d(&map_b, b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
-                                     static_cast<uint64_t>(num_groups) * N, K, ldb, BN, BK);
+                                     static_cast<uint64_t>(num_groups) * N, K, ldb, pairs ? BN_HALF : BN, BK);
     else rc = fsb_make_tmap_2d(&map_b, b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                                static_cast<uint64_t>(num_groups) * K, N, ldb, BK, 64);
     if (rc != FSB_OK) return rc;
@@ -1184,9 +1268,14 @@ FSB_API int fsb_gemm_bf16_grouped(const void* a, const void* b, void* d, int mod
   args.accumulate = accumulate; args.group_mode = mode; args.num_groups = num_groups;
   args.tile_expert = tile_expert; args.num_mtiles = num_mtiles; args.group_offs = group_offs;
   args.status = status;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return FSB_ERR_BAD_ARG;
+  if (pairs) {
+    const long long tiles2 = static_cast<long long>((args.M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) *
+                             (mode == 2 ? num_groups : 1) + (mode == 1 ? static_cast<long long>(num_groups) * ((N + BN - 1) / BN) : 0);
+    if (tiles2 >= (1ll << 31)) return FSB_ERR_TOO_LARGE;
+    const int clusters = tiles2 < g_pair_clusters[dev] ? static_cast<int>(tiles2) : g_pair_clusters[dev];
+    gemm_bf16_2sm_kernel<kGrouped><<<2 * clusters, NUM_THREADS, SMEM2_GROUPED_BYTES, stream>>>(map_a, map_b, args);
+    return cudaGetLastError() == cudaSuccess ? FSB_OK : FSB_ERR_LAUNCH;
+  }
   static bool attr_set[64] = {false};
   if (!attr_set[dev]) {
     if (cudaFuncSetAttribute(gemm_bf16_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,

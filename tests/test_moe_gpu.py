@@ -100,3 +100,34 @@ def test_latent_attention_operands_match_the_torch_steps(B, S, H, nope, rope, va
         # the reference rotates in fp32 (2^-22 of |x| + |y| < 2^3 H) on double inputs; one rounding to bf16 on top
         assert ((got - ref).abs() <= ref.abs() * 2.0 ** -8 + H * 2.0 ** -18).all()
     ops.check_status()
+
+
+@pytest.mark.parametrize("counts,D,F,dtype", [([0, 700, 1, 0, 513, 256, 1200, 0], 512, 320, torch.bfloat16),
+                                              ([385, 130, 900, 0], 264, 640, torch.float32), ([3000], 256, 256, torch.bfloat16)])
+def test_grouped_products_on_sm_pairs(counts, D, F, dtype):
+    """Groups of an odd number of 128-row tiles, empty groups at both ends, widths that no tile divides; each product
+    against fp64 on the same bf16 operands (fp32 sums of at most 1280 terms, one rounding)."""
+    torch.manual_seed(4)
+    dev = torch.device("cuda")
+    E = len(counts)
+    idx = torch.cat([torch.full((c,), e) for e, c in enumerate(counts)])[torch.randperm(sum(counts))].view(-1, 1).to(dev)
+    plan = moe.plan_routes(idx, E)
+    x = moe.moe_dispatch(torch.randn(idx.shape[0], D, device=dev).bfloat16(), plan).requires_grad_()
+    w = torch.randn(E, F, D, device=dev).bfloat16().requires_grad_()
+    if dtype == torch.float32:
+        w.main_grad, w.main_grad_written = torch.zeros(E, F, D, device=dev), False
+    y = moe.grouped_linear(x, w, plan)
+    offs = plan.offs.tolist()
+    dy = torch.zeros_like(y)
+    dy[:offs[-1]] = torch.randn(offs[-1], F, device=dev).bfloat16()
+    y.backward(dy)
+    ops.check_status()
+    dw = w.main_grad if dtype == torch.float32 else w.grad
+    for e in range(E):
+        r = slice(offs[e], offs[e + 1])
+        xe, we, de = x.detach()[r].double(), w.detach()[e].double(), dy[r].double()
+        pairs = [(dw[e], de.t() @ xe, de.abs().t() @ xe.abs())]
+        pairs += [(y[r], xe @ we.t(), xe.abs() @ we.abs().t()), (x.grad[r], de @ we, de.abs() @ we.abs())]
+        for got, ref, mag in pairs:
+            bound = mag * (1280 * 2.0 ** -24) + ref.abs() * (2.0 ** -8 if got.dtype == torch.bfloat16 else 0)
+            assert ((got.double() - ref).abs() <= bound).all()
