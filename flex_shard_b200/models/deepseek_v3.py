@@ -21,6 +21,7 @@ import torch.nn.functional as F
 
 from ..ops import elementwise as ew
 from ..ops import moe as moe_ops
+from ..ops.embedding import TokenEmbedding
 from ..ops.gemm import linear
 from ..ops.mla import mla_operands
 
@@ -239,7 +240,7 @@ class DeepSeekV3(nn.Module):
     def __init__(self, cfg: DeepSeekV3Config, dtype=torch.bfloat16, device=None):
         super().__init__()
         self.cfg = cfg
-        self.tok_embeddings = nn.Embedding(cfg.vocab_size, cfg.d_model, dtype=dtype, device=device)
+        self.tok_embeddings = TokenEmbedding(cfg.vocab_size, cfg.d_model, dtype=dtype, device=device)
         self.layers = nn.ModuleList([Block(cfg, i, dtype, device) for i in range(cfg.n_layers)])
         self.norm = nn.Parameter(torch.empty(cfg.d_model, dtype=dtype, device=device))
         self.output = nn.Parameter(torch.empty(cfg.vocab_size, cfg.d_model, dtype=dtype, device=device))

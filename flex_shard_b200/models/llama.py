@@ -18,6 +18,7 @@ import torch.nn as nn
 
 from ..ops import elementwise as ew
 from ..ops.attention import qkv_attention
+from ..ops.embedding import TokenEmbedding
 from ..ops.gemm import linear
 
 
@@ -101,7 +102,7 @@ class Llama(nn.Module):
     def __init__(self, cfg: LlamaConfig, dtype=torch.bfloat16, device=None):
         super().__init__()
         self.cfg = cfg
-        self.tok_embeddings = nn.Embedding(cfg.vocab_size, cfg.d_model, dtype=dtype, device=device)
+        self.tok_embeddings = TokenEmbedding(cfg.vocab_size, cfg.d_model, dtype=dtype, device=device)
         self.layers = nn.ModuleList([LlamaBlock(cfg, dtype, device) for _ in range(cfg.n_layers)])
         self.head = LlamaHead(cfg, dtype, device)
         self._rope = None

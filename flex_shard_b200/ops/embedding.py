@@ -1,0 +1,81 @@
+"""Token embedding whose weight gradient is written once, into the reduction bucket where the weight has one.
+
+The forward is PyTorch's gather. The backward (``csrc/embedding.cu``) adds the output gradients of equal tokens in fp32 and
+in token order, straight into the weight's ``main_grad`` view or a new gradient. Other weights (CPU, other dtypes, widths)
+take PyTorch's backward.
+"""
+from __future__ import annotations
+
+import torch
+import torch.nn as nn
+import torch.nn.functional as F
+
+from . import _lib
+from ._lib import count_launch
+
+_declared = False
+
+
+def _ensure():
+    global _declared
+    if not _declared:
+        import ctypes as c
+
+        vp, i32, i64 = c.c_void_p, c.c_int, c.c_longlong
+        _lib.declare("fsb_embedding_grad", [vp, vp, i32, i64, i32, i32, vp, i32, i32, vp, vp])
+        _declared = True
+
+
+def _write_grad(dy, tokens, out, accumulate: bool) -> None:
+    _ensure()
+    V, D = out.shape
+    T = tokens.numel()
+    scratch = torch.empty(3 * V + T + 1, dtype=torch.int32, device=dy.device)
+    rc = _lib.load().fsb_embedding_grad(dy.data_ptr(), tokens.data_ptr(), int(tokens.dtype == torch.int64), T, V, D,
+                                        out.data_ptr(), int(out.dtype == torch.float32), int(accumulate),
+                                        scratch.data_ptr(), _lib.stream_ptr(dy.device))
+    _lib.check(rc, "fsb_embedding_grad")
+    count_launch(4)
+
+
+class _Embedding(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, tokens, weight):
+        ctx.save_for_backward(tokens)
+        ctx.weight = weight      # its gradient destination is looked up when the gradient is there; its values are not needed
+        return F.embedding(tokens, weight)
+
+    @staticmethod
+    def backward(ctx, dy):
+        (tokens,), weight = ctx.saved_tensors, ctx.weight
+        if not ctx.needs_input_grad[1]:
+            return None, None
+        tokens = tokens.reshape(-1).contiguous()
+        dy = dy.reshape(-1, dy.shape[-1]).contiguous()
+        if dy.data_ptr() % 16:
+            dy = dy.clone()
+        main = getattr(weight, "main_grad", None)
+        if (isinstance(main, torch.Tensor) and main.dtype == torch.float32 and main.is_contiguous()
+                and main.shape == weight.shape and main.data_ptr() % 16 == 0):
+            _write_grad(dy, tokens, main, bool(getattr(weight, "main_grad_written", False)))
+            weight.main_grad_written = True
+            return None, None
+        dw = torch.empty(weight.shape, dtype=weight.dtype, device=weight.device)
+        _write_grad(dy, tokens, dw, False)
+        return None, dw
+
+
+def embedding(tokens, weight):
+    """Rows ``tokens`` (any shape, int32 or int64) of ``weight`` [V, D]."""
+    if (weight.is_cuda and weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.shape[1] % 8 == 0
+            and 0 < weight.shape[1] <= 8192 and weight.shape[0] > 0 and 0 < tokens.numel() < 2 ** 31
+            and tokens.device == weight.device and tokens.dtype in (torch.int32, torch.int64)):
+        return _Embedding.apply(tokens, weight)
+    return F.embedding(tokens, weight)
+
+
+class TokenEmbedding(nn.Embedding):
+    """``nn.Embedding`` (without padding row, norm limit or sparse gradients) on ``embedding``."""
+
+    def forward(self, tokens):
+        return embedding(tokens, self.weight)

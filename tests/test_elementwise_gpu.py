@@ -188,3 +188,38 @@ def test_cross_entropy_gradient_of_a_scaled_loss(shape, factor):
         torch.testing.assert_close(got.double(), ref.grad, rtol=2.0 ** -7, atol=2.0 ** -12 / shape[0])
     assert torch.equal(again, twice)
     ops.check_status()
+
+
+@pytest.mark.parametrize("T,V,D,kind", [(1, 3, 8, "any"), (300, 50, 264, "any"), (5000, 7, 2056, "one"), (4097, 4000, 4096, "any"),
+                                        (2048, 100, 8192, "one"), (777, 1, 64, "any")])
+@pytest.mark.parametrize("main", [None, False, True])
+def test_embedding_gradient(T, V, D, kind, main):
+    """Values read once, never, and more often than a block orders at a time; a new bf16 gradient, an fp32 destination that
+    is overwritten (main False) or added to (main True)."""
+    from flex_shard_b200.ops.embedding import embedding
+
+    torch.manual_seed(13)
+    w = torch.randn(V, D, device=DEV).bfloat16().requires_grad_()
+    tokens = torch.randint(0, V, (T,), device=DEV) if kind == "any" else torch.full((T,), V - 1, device=DEV)
+    if T % 2:
+        tokens = tokens.int()
+    dy = torch.randn(T, D, device=DEV).bfloat16()
+    got = []
+    for _ in range(2):
+        base = torch.randn(V, D, device=DEV, generator=torch.Generator(DEV).manual_seed(1))
+        w.grad = None
+        if main is not None:
+            w.main_grad, w.main_grad_written = base.clone(), main
+        y = embedding(tokens.view(1, -1), w)
+        assert torch.equal(y[0], w.detach()[tokens])
+        y.backward(dy[None])
+        got.append(w.grad if main is None else w.main_grad)
+    ops.check_status()
+    assert torch.equal(*got)                                          # the same bits on every run
+    want = torch.zeros(V, D, device=DEV, dtype=torch.float64).index_add_(0, tokens.long(), dy.double())
+    mag = torch.zeros_like(want).index_add_(0, tokens.long(), dy.double().abs())
+    if main:
+        want, mag = want + base.double(), mag + base.double().abs()
+    count = torch.bincount(tokens, minlength=V).clamp_min(1)[:, None]
+    bound = mag * (count * 2.0 ** -23) + (want.abs() * 2.0 ** -8 if main is None else 0)
+    assert ((got[0].double() - want).abs() <= bound).all()
