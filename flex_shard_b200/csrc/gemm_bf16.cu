@@ -164,6 +164,14 @@ __device__ __forceinline__ TileInfo get_tile(const GemmArgs& args, int tile, int
   return t;
 }
 
+// 32 bytes (one sector) in one store; p on a 32-byte boundary. A lane of the epilogue owns a row, so with 16-byte stores
+// every sector of D was written in two halves by two instructions.
+__device__ __forceinline__ void store32(void* p, const uint32_t (&w)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+               "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
+
 // Epilogue of one 128 x 256 accumulator tile: the calling warp owns TMEM lanes [32*quarter, +32)
 // (t_row = TMEM address of its lane quarter, column 0 of the accumulator) = rows
 // tm*128 + 32*quarter + lane of D. `stg` is the warp's padded 32x32 fp32 staging tile. `mirror`: D is symmetric and
@@ -182,10 +190,27 @@ __device__ __forceinline__ void store_tile(const GemmArgs& args, long long d_row
     d_base = args.d_peer[row / args.d_block_rows];
     d_off = (row % args.d_block_rows) * args.ldd;
   }
+  // A bf16 addend on the 16-byte grid is fetched one chunk of 32 columns ahead: one element at a time, the 32 lanes of a
+  // warp (32 different rows) cost 32 sectors per load, and fetched when needed its latency came eight times per tile
+  // (2048 x 2048 tile grids of one wave: 3.7 us of a 21.5 us product).
+  const __nv_bfloat16* c_row = static_cast<const __nv_bfloat16*>(args.c) + (d_row_off + row) * args.ldc + tn * BN;
+  const bool c_ahead = args.c != nullptr && !args.c_fp32 && row_ok && (reinterpret_cast<uintptr_t>(c_row) & 15) == 0;
+  uint4 c_next[4];
+  auto fetch_addend = [&](int c0) {
+    if (c_ahead && c0 < BN && tn * BN + c0 + 32 <= args.N) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) c_next[i] = reinterpret_cast<const uint4*>(c_row + c0)[i];
+    }
+  };
+  fetch_addend(0);
 #pragma unroll 1
   for (int c0 = 0; c0 < BN; c0 += 32) {
     const int col = tn * BN + c0;
     if (col >= args.N) break;  // uniform across the warp
+    uint4 c_raw[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c_raw[i] = c_next[i];
+    fetch_addend(c0 + 32);
     uint32_t r[32];
     tmem_ld_32x32(t_row + c0, r);
     tmem_ld_wait();
@@ -209,61 +234,75 @@ __device__ __forceinline__ void store_tile(const GemmArgs& args, long long d_row
       __syncwarp();
       continue;
     }
-    if (row_ok) {
-      float v[32];
+    float v[32];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * args.alpha;
-      const bool full = (col + 32 <= args.N);
-      if (args.c != nullptr) {
-        // The addend's row of 32 values in 16-byte pieces where its alignment allows: one element at a time, the 32
-        // lanes of a warp (32 different rows) cost 32 sectors per load and the addend took longer than the product's
-        // main loop. With the mirrored store below in place of a pass of its own over D, one Muon step over the four
-        // matrices of a 4096 / 14336 decoder layer went from 17.0 to 14.3 ms.
-        const long long c_off = (d_row_off + row) * args.ldc + col;
-        if (args.c_fp32) {
-          const float* cp = static_cast<const float*>(args.c) + c_off;
-          if (full && (reinterpret_cast<uintptr_t>(cp) & 15) == 0) {
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * args.alpha;
+    const bool full = (col + 32 <= args.N);
+    if (args.c != nullptr && row_ok) {
+      if (args.c_fp32) {
+        const float* cp = static_cast<const float*>(args.c) + (d_row_off + row) * args.ldc + col;
+        if (full && (reinterpret_cast<uintptr_t>(cp) & 15) == 0) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              const float4 f = *reinterpret_cast<const float4*>(cp + i);
-              v[i] += args.beta * f.x;
-              v[i + 1] += args.beta * f.y;
-              v[i + 2] += args.beta * f.z;
-              v[i + 3] += args.beta * f.w;
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (full || col + i < args.N) v[i] += args.beta * cp[i];
+          for (int i = 0; i < 32; i += 4) {
+            const float4 f = *reinterpret_cast<const float4*>(cp + i);
+            v[i] += args.beta * f.x;
+            v[i + 1] += args.beta * f.y;
+            v[i + 2] += args.beta * f.z;
+            v[i + 3] += args.beta * f.w;
           }
         } else {
-          const __nv_bfloat16* cp = static_cast<const __nv_bfloat16*>(args.c) + c_off;
-          if (full && (reinterpret_cast<uintptr_t>(cp) & 15) == 0) {
-            uint4 raw[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) raw[i] = reinterpret_cast<const uint4*>(cp)[i];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const float2 f = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(raw)[i >> 1]);
-              v[i] += args.beta * ((i & 1) ? f.y : f.x);
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (full || col + i < args.N) v[i] += args.beta * __bfloat162float(cp[i]);
-          }
+          for (int i = 0; i < 32; ++i)
+            if (full || col + i < args.N) v[i] += args.beta * cp[i];
         }
-      }
-      if (mirror) {
-        // the element below the diagonal that equals this one: 32 lanes write 64 contiguous bytes of row col + i
-        __nv_bfloat16* mp = static_cast<__nv_bfloat16*>(args.d) + (d_row_off + col) * args.ldd + row;
+      } else if (full && c_ahead) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const float2 f = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(c_raw)[i >> 1]);
+          v[i] += args.beta * ((i & 1) ? f.y : f.x);
+        }
+      } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i)
-          if (full || col + i < args.N) mp[i * args.ldd] = __float2bfloat16(v[i]);
+          if (full || col + i < args.N) v[i] += args.beta * __bfloat162float(c_row[c0 + i]);
       }
+    }
+    if (mirror) {
+      // The elements below the diagonal that equal these: the warp's 32 x 32 block is transposed through shared memory,
+      // so that a lane stores 64 contiguous bytes of row col + lane. (A two-byte store per element, 32 lanes to a row,
+      // took 7 us a tile: more than the main loop over a depth of 1024.)
+#pragma unroll
+      for (int i = 0; i < 32; ++i) stg[lane * 33 + i] = v[i];
+      __syncwarp();
+      const long long row0 = static_cast<long long>(tm) * BM + quarter * 32;
+      if (col + lane < args.N && row0 < args.M) {
+        __nv_bfloat16* mp = static_cast<__nv_bfloat16*>(args.d) + (d_row_off + col + lane) * args.ldd + row0;
+        if (row0 + 32 <= args.M && (reinterpret_cast<uintptr_t>(mp) & 31) == 0) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 16) {
+            uint32_t w[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) w[j] = pack_bf16x2(stg[(i + 2 * j) * 33 + lane], stg[(i + 2 * j + 1) * 33 + lane]);
+            store32(mp + i, w);
+          }
+        } else {
+          for (int i = 0; i < 32 && row0 + i < args.M; ++i) mp[i] = __float2bfloat16(stg[i * 33 + lane]);
+        }
+      }
+      __syncwarp();
+    }
+    if (row_ok) {
       if (args.d_fp32) {
         float* dp = static_cast<float*>(d_base) + d_off + col;
-        if (full && (args.ldd % 4 == 0) && (args.d_block_stride % 4 == 0)) {
+        if (full && !args.accumulate && (reinterpret_cast<uintptr_t>(dp) & 31) == 0) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 8) {
+            uint32_t w[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) w[j] = __float_as_uint(v[i + j]);
+            store32(dp + i, w);
+          }
+        } else if (full && (args.ldd % 4 == 0) && (args.d_block_stride % 4 == 0)) {
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
             float4 o = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
@@ -279,7 +318,15 @@ __device__ __forceinline__ void store_tile(const GemmArgs& args, long long d_row
         }
       } else {
         __nv_bfloat16* dp = static_cast<__nv_bfloat16*>(d_base) + d_off + col;
-        if (full && (args.ldd % 8 == 0) && (args.d_block_stride % 8 == 0)) {
+        if (full && !args.accumulate && (reinterpret_cast<uintptr_t>(dp) & 31) == 0) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 16) {
+            uint32_t w[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) w[j] = pack_bf16x2(v[i + 2 * j], v[i + 2 * j + 1]);
+            store32(dp + i, w);
+          }
+        } else if (full && (args.ldd % 8 == 0) && (args.d_block_stride % 8 == 0)) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
             if (args.accumulate) {
@@ -1180,8 +1227,8 @@ static int gemm_pair_launch(const void* a, const void* b, void* d, const void* c
 // Bound by the tensor cores for stacks of expert matrices, by latency for a stack of attention heads (a 192 x 1536
 // matrix is a single tile, so one grid takes the whole stack). A Muon step over 64 experts of 2816 x 2048 and of
 // 2048 x 1408, 64 attention-head matrices and the ten single matrices of two blocks: 64.7 ms with the one-SM grouped
-// kernel (full products, heads one at a time), 28.8 ms here, 18.4 ms of them in this kernel (about 1 180 TFLOP/s of
-// executed products).
+// kernel (full products, heads one at a time), 26.6 ms here, 16.9 ms of them in this kernel (about 1 300 TFLOP/s of
+// executed products; 20.3 ms while the mirrored half was stored two bytes at a time).
 FSB_API int fsb_gemm_bf16_batched(const void* a, const void* b, void* d, const void* c, int count, int M, int N, int K,
                                   int a_mn, int b_mn, float alpha, float beta, int symmetric, int* status,
                                   cudaStream_t stream) {
