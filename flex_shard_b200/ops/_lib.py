@@ -93,6 +93,7 @@ def _declare(lib) -> None:
         "fsb_rmsnorm_fwd": [vp, vp, vp, vp, vp, vp, i64, i32, f32, vp],
         "fsb_rmsnorm_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i64, i32, vp],
         "fsb_rope": [vp, vp, i64, i32, i32, i32, i64, i32, vp],
+        "fsb_rope_bwd_from_acc": [vp, vp, vp, i64, i32, i32, i32, i32, i64, vp],
         "fsb_swiglu_fwd": [vp, vp, i64, i32, vp],
         "fsb_swiglu_bwd": [vp, vp, vp, i64, i32, vp],
         "fsb_cross_entropy": [vp, vp, vp, i64, i32, i64, f32, i64, vp],

@@ -115,11 +115,8 @@ class _QKVAttention(torch.autograd.Function):
             ctx.dims = (B, S, Hq, Hkv)
             return o.detach().to(qkv.dtype).reshape(B, S, Hq * HD)
         assert qkv.dtype == torch.bfloat16 and qkv.is_contiguous()
-        q = qkv[..., : Hq * HD].view(B, S, Hq, HD)
-        k = qkv[..., Hq * HD: (Hq + Hkv) * HD].view(B, S, Hkv, HD)
-        if rope_table is not None:
-            _rope_inplace(q, rope_table, False)
-            _rope_inplace(k, rope_table, False)
+        if rope_table is not None:   # query and key heads are neighbours: one launch
+            _rope_inplace(qkv[..., : (Hq + Hkv) * HD].view(B, S, Hq + Hkv, HD), rope_table, False)
         o = torch.empty(B, S, Hq * HD, dtype=qkv.dtype, device=qkv.device)
         lse = torch.empty(B, Hq, S, dtype=torch.float32, device=qkv.device)
         base = qkv.data_ptr()
@@ -163,12 +160,14 @@ class _QKVAttention(torch.autograd.Function):
                               dbase + Hq * HD * 2, dbase + (Hq + Hkv) * HD * 2, B, S, Hq, Hkv,
                               C, C, C, Hq * HD, Hq * HD, C, C, scale, status.data_ptr(), _lib.stream_ptr(dev))
         _lib.check(rc, "fsb_attn_bwd")
-        rc = lib.fsb_cast2d_f32_bf16(dq_acc.data_ptr(), dbase, B * S, Hq * HD, Hq * HD, C, _lib.stream_ptr(dev))
-        _lib.check(rc, "fsb_cast2d_f32_bf16")
+        if rope_table is not None:   # the query gradient is rounded and both are rotated back in one pass
+            rc = lib.fsb_rope_bwd_from_acc(dbase, dq_acc.data_ptr(), rope_table.data_ptr(), B * S, S, Hq, Hkv, HD, C,
+                                           _lib.stream_ptr(dev))
+            _lib.check(rc, "fsb_rope_bwd_from_acc")
+        else:
+            rc = lib.fsb_cast2d_f32_bf16(dq_acc.data_ptr(), dbase, B * S, Hq * HD, Hq * HD, C, _lib.stream_ptr(dev))
+            _lib.check(rc, "fsb_cast2d_f32_bf16")
         count_launch(4)
-        if rope_table is not None:
-            _rope_inplace(dqkv[..., : Hq * HD].view(B, S, Hq, HD), rope_table, True)
-            _rope_inplace(dqkv[..., Hq * HD: (Hq + Hkv) * HD].view(B, S, Hkv, HD), rope_table, True)
         return dqkv, None, None, None
 
 
