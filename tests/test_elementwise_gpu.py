@@ -223,3 +223,26 @@ def test_embedding_gradient(T, V, D, kind, main):
     count = torch.bincount(tokens, minlength=V).clamp_min(1)[:, None]
     bound = mag * (count * 2.0 ** -23) + (want.abs() * 2.0 ** -8 if main is None else 0)
     assert ((got[0].double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("V", [56320, 56328, 102400, 145408, 145416])
+def test_cross_entropy_of_rows_on_either_side_of_the_splits(V):
+    """Rows of one CTA, of a pair of CTAs (odd halves, the largest) and too long to stay on chip; targets in both halves,
+    ignored ones, and a maximum far above the rest in either half."""
+    torch.manual_seed(6)
+    T = 9
+    x = torch.randn(T, V, device=DEV).bfloat16()
+    x[0, 5], x[1, V - 3] = 60.0, 60.0
+    tgt = torch.randint(0, V, (T,), device=DEV)
+    tgt[2], tgt[3], tgt[4] = 0, V - 1, -100
+    tgt[5], tgt[6] = (V // 8 + 1) // 2 * 8 - 1, (V // 8 + 1) // 2 * 8
+    ref = x.double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(ref, tgt, reduction="sum") / T
+    want.backward()
+    got_x = x.clone().requires_grad_()
+    loss = ew.cross_entropy(got_x * 1.0, tgt)
+    loss.backward()
+    # fp32 sums over V terms and the fast exponential (2 ulp of an argument of up to 70): 1e-5; one rounding to bf16
+    assert abs(float(loss.detach()) - float(want.detach())) <= 1e-5 * abs(float(want.detach()))
+    torch.testing.assert_close(got_x.grad.double(), ref.grad, rtol=2.0 ** -8 + 2e-5, atol=1e-9)
+    ops.check_status()
