@@ -279,8 +279,9 @@ class _CrossEntropy(torch.autograd.Function):
             return dlogits, None, None, None, None
         if (dlogits.is_cuda and dlogits.is_contiguous() and dlogits.data_ptr() % 16 == 0 and dlogits.dtype == torch.bfloat16
                 and dloss.device == dlogits.device and dloss.dtype == torch.float32
-                and not torch._C._autograd._get_current_graph_task_keep_graph()):
-            # this graph is not run again, so its saved tensor can be scaled in place (a no-op when the gradient is 1)
+                and not torch._C._autograd._get_current_graph_task_keep_graph() and not torch.is_grad_enabled()):
+            # this graph is not run or differentiated again, so its saved tensor can be scaled in place (a no-op when the
+            # gradient is 1)
             rc = _lib.load().fsb_scale_by_scalar(dlogits.data_ptr(), dloss.data_ptr(), dlogits.numel(),
                                                  _s(dlogits.device))
             _lib.check(rc, "fsb_scale_by_scalar")

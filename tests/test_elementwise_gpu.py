@@ -183,7 +183,10 @@ def test_cross_entropy_gradient_of_a_scaled_loss(shape, factor):
     again = torch.autograd.grad(loss, leaf, retain_graph=True)[0].clone()
     twice = torch.autograd.grad(loss, leaf, retain_graph=True)[0].clone()
     last = torch.autograd.grad(loss, leaf)[0]
-    for got in (again, twice, last):
+    scaled = torch.full((), factor, device=DEV, requires_grad=True)       # a gradient that is differentiated again
+    graph = torch.autograd.grad(ew.cross_entropy(leaf.clone(), target) * scaled, leaf, create_graph=True, retain_graph=False)[0]
+    assert graph.requires_grad
+    for got in (again, twice, last, graph.detach()):
         # two roundings to bf16 (the saved gradient, its scaled copy) of values below 1 / T
         torch.testing.assert_close(got.double(), ref.grad, rtol=2.0 ** -7, atol=2.0 ** -12 / shape[0])
     assert torch.equal(again, twice)
