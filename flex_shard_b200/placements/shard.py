@@ -368,11 +368,14 @@ class Shard(Placement):
         """On one rank, gradients that would be widened to the reduce dtype and rounded back to the dtype they already
         have come out as they went in: no packing, no cast. (Gradients that stay in the reduce dtype are packed: the
         optimizer then takes the bucket as one flat launch.) One expert block and its vocabulary, 1.07 G parameters in
-        bf16 reduced in fp32: 2.6 ms of a training step for the two passes."""
+        bf16 reduced in fp32: 2.6 ms of a training step for the two passes.
+
+        Each must be alone in its memory: autograd gives the addends of a sum, or a parameter whose view is the output,
+        views of one storage, and what is handed on is later added to and scaled in place."""
         return all(g.dtype != reduce_dtype and g.dtype == (i.grad_dtype or i.storage_dtype)
                    and torch.promote_types(g.dtype, reduce_dtype) == reduce_dtype and g.is_contiguous()
                    and tuple(g.shape) == tuple(i.local_shape) and getattr(g, "_fsb_bucket", None) is None
-                   for i, g in zip(infos, grads))
+                   and _alone_in_its_memory(g) for i, g in zip(infos, grads))
 
     def _pack_grads(self, infos, grads, W, reduce_dtype, offs, row):
         needs_zero = any(info.global_shape[info.placement.dim] % W != 0 for info in infos)
@@ -456,6 +459,15 @@ class Shard(Placement):
             ln = info.local_numel
             grads.append(out[o:o + ln].view(info.local_shape) if ln > 0 else out[o:o].view(info.local_shape))
         return PlacementReduceGradResult(grads=grads, output=out)
+
+
+def _alone_in_its_memory(t) -> bool:
+    """Whether no other tensor, wherever it is held, shares ``t``'s storage, and ``t`` takes all of it."""
+    if type(t) is not torch.Tensor:
+        return False
+    storage = t.untyped_storage()
+    # two holders: the tensor and the Python object made here
+    return storage.nbytes() == t.numel() * t.element_size() and torch._C._storage_Use_Count(storage._cdata) == 2
 
 
 def shard_placement_fn(dim: int = 0, grad_bucket: bool = False):

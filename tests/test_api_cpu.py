@@ -379,3 +379,73 @@ def test_one_rank_reduction_equals_the_packed_one(storage, reduce, factor, monke
         res.append([p.grad for p in m.parameters()])
     for a, b in zip(*res):
         assert a.dtype == b.dtype == storage and torch.equal(a, b)
+
+
+class TwoSums(nn.Module):
+    """Autograd gives the addends of a sum gradients that are views of one storage."""
+
+    def __init__(self):
+        super().__init__()
+        self.pos, self.typ, self.far = (nn.Parameter(torch.randn(6, 8).bfloat16()) for _ in range(3))
+
+    def forward(self, x):
+        return x + (self.pos.unsqueeze(0) + self.typ.unsqueeze(0)) + self.far.view(1, 6, 8)
+
+
+@pytest.mark.parametrize("buckets", [[["*"]], [["pos"], ["typ"], ["far"]]])
+def test_gradients_that_share_memory_are_taken_apart(buckets, monkeypatch):
+    """On one rank, gradients that are views of one storage, or of the tensor handed to ``backward``, are packed: over
+    three accumulated backward passes and a clip each parameter has the gradient that it has when all are packed, no two
+    share memory, and the caller's tensor stays as it was."""
+    from flex_shard_b200 import BucketSpec, MixedPrecisionPolicy, flex_shard
+    from flex_shard_b200.placements.shard import Shard
+    from flex_shard_b200.utils.training import clip_grad_norm_
+
+    mp = MixedPrecisionPolicy(param_dtype=torch.bfloat16, reduce_dtype=torch.float32)
+    res = []
+    for packed in (False, True):
+        if packed:
+            monkeypatch.setattr(Shard, "_reduces_to_itself", staticmethod(lambda *a: False))
+        torch.manual_seed(0)
+        m = TwoSums()
+        flex_shard(m, [BucketSpec(b, mp_policy=mp) for b in buckets])
+        got = []
+        dy = torch.randn(1, 6, 8, generator=torch.Generator().manual_seed(1)).bfloat16()
+        kept = dy.clone()
+        for _ in range(3):
+            m(torch.zeros(1, 6, 8).bfloat16()).backward(dy)
+            got.append([p.grad.clone() for p in m.parameters()])
+        got.append([clip_grad_norm_(m, 1.0)] + [p.grad.clone() for p in m.parameters()])
+        assert len({t.untyped_storage().data_ptr() for t in (dy, *(p.grad for p in m.parameters()))}) == 4
+        assert torch.equal(dy, kept)
+        res.append(sum(got, []))
+    for a, b in zip(*res):
+        assert torch.equal(a, b)
+
+
+class Sliced(nn.Module):
+    def __init__(self):
+        super().__init__()
+        self.w = nn.Parameter(torch.randn(4, 8).bfloat16())
+
+    def forward(self, x):
+        return torch.cat([self.w, x])
+
+
+def test_a_gradient_does_not_keep_a_larger_tensor_alive(monkeypatch):
+    """... and gradients that are tensors of their own are still handed on."""
+    from flex_shard_b200 import BucketSpec, MixedPrecisionPolicy, flex_shard
+    from flex_shard_b200.placements.shard import Shard
+
+    mp = MixedPrecisionPolicy(param_dtype=torch.bfloat16, reduce_dtype=torch.float32)
+    seen, rule = [], Shard._reduces_to_itself
+    monkeypatch.setattr(Shard, "_reduces_to_itself", staticmethod(lambda *a: seen.append(rule(*a)) or seen[-1]))
+    m = Net().bfloat16()
+    flex_shard(m, [BucketSpec(["a.*"], mp_policy=mp), BucketSpec(["b.*"], mp_policy=mp)])
+    m(torch.randn(5, 8).bfloat16()).square().sum().backward()
+    assert seen == [True, True]
+    m = Sliced()
+    flex_shard(m, [BucketSpec(["*"], mp_policy=mp)])
+    m(torch.zeros(60, 8).bfloat16()).backward(torch.ones(64, 8).bfloat16())
+    g = m.w.grad
+    assert g.untyped_storage().nbytes() == g.numel() * g.element_size()
