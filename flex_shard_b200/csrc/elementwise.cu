@@ -419,6 +419,7 @@ cross_entropy_resident_kernel(__nv_bfloat16* __restrict__ logits, const long lon
   extern __shared__ __align__(16) uint4 rowv[];
   __shared__ float red[32];
   __shared__ float other[2];   // (max, sum) of the other half
+  if constexpr (PAIR) cluster_arrive();   // waited for before the exchange: the row's load hides it
   const float L2E = 1.4426950408889634f;
   const long long row = PAIR ? blockIdx.x >> 1 : blockIdx.x;
   const int part = PAIR ? static_cast<int>(cluster_ctarank()) : 0;
@@ -469,11 +470,13 @@ cross_entropy_resident_kernel(__nv_bfloat16* __restrict__ logits, const long lon
   float mx = block_max<CE_THREADS>(m, red);
   float se = block_sum<CE_THREADS>(m == -INFINITY ? 0.f : s * exp2f((m - mx) * L2E), red);
   if constexpr (PAIR) {
+    cluster_wait();       // the other CTA has started, so its shared memory may be written
     if (tid == 0) {
       const uint32_t dst = map_to_cta(smem_u32(other), part ^ 1);
       asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(mx) : "memory");
       asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + 4), "f"(se) : "memory");
     }
+    __syncwarp();
     cluster_sync_all();   // both halves have written; each reads only its own shared memory from here on
     const float mo_ = other[0], so = other[1], both = fmaxf(mx, mo_);
     const float mine = mx == -INFINITY ? 0.f : se * exp2f((mx - both) * L2E);
