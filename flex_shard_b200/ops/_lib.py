@@ -125,6 +125,12 @@ def stream_ptr(device=None) -> int:
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
+def plain(*tensors) -> bool:
+    """Whether a kernel may be given these tensors' addresses: no subclasses, and no tensors without memory of their own
+    (those that ``vmap``, batched gradients and the ``torch.func`` transforms hand to an operator)."""
+    return all(type(t) in (torch.Tensor, torch.nn.Parameter) and torch._C._has_storage(t) for t in tensors)
+
+
 STATUS_INTS = 8     # [0] code; a failed peer wait also leaves [1],[2] flag address, [3] epoch, [4] peer, [5] value seen
 
 

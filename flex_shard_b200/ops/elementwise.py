@@ -277,9 +277,7 @@ class _CrossEntropy(torch.autograd.Function):
         (dlogits,) = ctx.saved_tensors
         if ctx.unit_grad:
             return dlogits, None, None, None, None
-        if (dlogits.is_cuda and dlogits.is_contiguous() and dlogits.data_ptr() % 16 == 0 and dlogits.dtype == torch.bfloat16
-                and dloss.device == dlogits.device and dloss.dtype == torch.float32
-                and not torch._C._autograd._get_current_graph_task_keep_graph() and not torch.is_grad_enabled()):
+        if _scaled_in_place(dlogits, dloss):
             # this graph is not run or differentiated again, so its saved tensor can be scaled in place (a no-op when the
             # gradient is 1)
             rc = _lib.load().fsb_scale_by_scalar(dlogits.data_ptr(), dloss.data_ptr(), dlogits.numel(),
@@ -288,6 +286,15 @@ class _CrossEntropy(torch.autograd.Function):
             count_launch()
             return dlogits, None, None, None, None
         return dlogits * dloss.to(dlogits.dtype), None, None, None, None
+
+
+def _scaled_in_place(dlogits, dloss) -> bool:
+    """Whether the saved gradient may be overwritten with its product: a kernel call on plain tensors (batched gradients
+    hand in a ``dloss`` without memory), in a backward whose graph is not kept and not differentiated."""
+    return (_lib.plain(dlogits, dloss) and dloss.dim() == 0
+            and dlogits.is_cuda and dlogits.is_contiguous() and dlogits.data_ptr() % 16 == 0
+            and dlogits.dtype == torch.bfloat16 and dloss.device == dlogits.device and dloss.dtype == torch.float32
+            and not torch._C._autograd._get_current_graph_task_keep_graph() and not torch.is_grad_enabled())
 
 
 def cross_entropy(logits, target, scale: float | None = None, ignore_index: int = -100,

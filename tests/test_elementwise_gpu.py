@@ -193,6 +193,19 @@ def test_cross_entropy_gradient_of_a_scaled_loss(shape, factor):
     ops.check_status()
 
 
+def test_cross_entropy_takes_batched_loss_gradients():
+    torch.manual_seed(3)
+    x, target = torch.randn(5, 1000, device=DEV).bfloat16(), torch.randint(0, 1000, (5,), device=DEV)
+    factors = torch.tensor([1.0, 0.37, -2.0], device=DEV)
+    ref = x.double().requires_grad_()
+    (want,) = torch.autograd.grad(torch.nn.functional.cross_entropy(ref, target), ref)
+    leaf = x.clone().requires_grad_()
+    (got,) = torch.autograd.grad(ew.cross_entropy(leaf.clone(), target), leaf, factors, is_grads_batched=True)
+    # three roundings to bf16: the saved gradient, the factor, their product
+    torch.testing.assert_close(got.double(), factors.double()[:, None, None] * want, rtol=3 * 2.0 ** -8, atol=2.0 ** -12)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("T,V,D,kind", [(1, 3, 8, "any"), (300, 50, 264, "any"), (5000, 7, 2056, "one"), (4097, 4000, 4096, "any"),
                                         (2048, 100, 8192, "one"), (777, 1, 64, "any")])
 @pytest.mark.parametrize("main", [None, False, True])
