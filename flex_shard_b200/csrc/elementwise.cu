@@ -534,7 +534,6 @@ scale_by_scalar_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ 
 // eps added after the sqrt), maximize=False, amsgrad=False.
 struct AdamArgs {
   float lr, beta1, beta2, eps, weight_decay, bias1, bias2_sqrt, grad_scale;
-  float step_size, inv_bias2_sqrt;   // lr / bias1, 1 / bias2_sqrt
 };
 __device__ __forceinline__ void ld8(const float* p, float (&f)[8]) {
   const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
@@ -562,37 +561,24 @@ __device__ __forceinline__ void st8_wide(float* p, const float (&f)[8]) {
 }
 __device__ __forceinline__ void st8_wide(__nv_bfloat16* p, const float (&f)[8]) { store8(p, f); }
 
-// APPROX: the square root and the two quotients of the update in single-instruction approximations (each within 2 ulp
-// of fp32). Only where the parameter is stored as bf16, whose rounding is 2^14 times coarser; moments are not
-// affected, an fp32 parameter keeps the IEEE sequences.
-template <bool APPROX>
 __device__ __forceinline__ void adamw_update(float& pv, float gv, float& mv, float& vv, const AdamArgs& a) {
   gv *= a.grad_scale;
   pv *= (1.f - a.lr * a.weight_decay);
   mv = mv + (1.f - a.beta1) * (gv - mv);  // lerp, as torch does
   vv = a.beta2 * vv + (1.f - a.beta2) * gv * gv;
-  if constexpr (APPROX) {
-    float root;
-    asm("sqrt.approx.f32 %0, %1;" : "=f"(root) : "f"(vv));
-    const float denom = root * a.inv_bias2_sqrt + a.eps;
-    pv -= a.step_size * __fdividef(mv, denom);
-  } else {
-    const float denom = sqrtf(vv) / a.bias2_sqrt + a.eps;
-    pv -= (a.lr / a.bias1) * (mv / denom);
-  }
+  const float denom = sqrtf(vv) / a.bias2_sqrt + a.eps;
+  pv -= (a.lr / a.bias1) * (mv / denom);
 }
 
-// 8 elements per thread per iteration; `n8` full groups, then a scalar tail. Bound by memory: 16 B of moments plus
-// parameter and gradient per element; at the clocks of a training step the IEEE square root and quotients (some 40
-// instructions an element) were as long as the memory traffic. A step over three 4096 / 14336 layers with an fp32
-// gradient: 67.7 -> 65.9 ms; one expert block: 23.1 -> 22.75 ms. WIDE: the fp32 arrays start on 32-byte boundaries (every flat bucket does) and
-// move in 32-byte accesses; otherwise 16-byte ones.
+// 8 elements per thread per iteration; `n8` full groups, then a scalar tail. Bound by memory (16 B of moments plus
+// parameter and gradient per element) as long as the SM clock is high; at the clocks of a training step the IEEE square
+// root and quotients, some 40 instructions an element, take about as long. WIDE: the fp32 arrays start on 32-byte
+// boundaries (every flat bucket does) and move in 32-byte accesses; otherwise 16-byte ones.
 template <typename PT, typename GT, bool WIDE>
 __global__ void __launch_bounds__(256)
 adamw_kernel(PT* __restrict__ p, const GT* __restrict__ g, float* __restrict__ m,
              float* __restrict__ v, __nv_bfloat16* __restrict__ p_lowp, long long n, int vec_ok,
              AdamArgs a) {
-  constexpr bool APPROX = std::is_same<PT, __nv_bfloat16>::value;
   const long long tid = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   const long long n8 = vec_ok ? n / 8 : 0;
@@ -610,7 +596,7 @@ adamw_kernel(PT* __restrict__ p, const GT* __restrict__ g, float* __restrict__ m
       ld8(v + i * 8, vf);
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) adamw_update<APPROX>(pf[j], gf[j], mf[j], vf[j], a);
+    for (int j = 0; j < 8; ++j) adamw_update(pf[j], gf[j], mf[j], vf[j], a);
     if constexpr (WIDE) {
       st8_wide(p + i * 8, pf);
       st8_wide(m + i * 8, mf);
@@ -624,7 +610,7 @@ adamw_kernel(PT* __restrict__ p, const GT* __restrict__ g, float* __restrict__ m
   }
   for (long long i = n8 * 8 + tid; i < n; i += stride) {
     float pv = static_cast<float>(p[i]), mv = m[i], vv = v[i];
-    adamw_update<APPROX>(pv, static_cast<float>(g[i]), mv, vv, a);
+    adamw_update(pv, static_cast<float>(g[i]), mv, vv, a);
     p[i] = static_cast<PT>(pv);
     m[i] = mv;
     v[i] = vv;
@@ -953,8 +939,6 @@ FSB_API int fsb_adamw(void* p, const void* g, float* m, float* v, void* p_lowp, 
   a.bias1 = 1.f - powf(beta1, static_cast<float>(step));
   a.bias2_sqrt = sqrtf(1.f - powf(beta2, static_cast<float>(step)));
   a.grad_scale = grad_scale;
-  a.step_size = a.lr / a.bias1;
-  a.inv_bias2_sqrt = 1.f / a.bias2_sqrt;
   const int grid = grid_for(n, 256, 8);
   __nv_bfloat16* lp = static_cast<__nv_bfloat16*>(p_lowp);
   const uintptr_t al = reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) |

@@ -1,4 +1,5 @@
 """Bandwidth kernels against fp32 PyTorch references (the CPU path of the same wrappers)."""
+import numpy as np
 import pytest
 import torch
 
@@ -139,6 +140,25 @@ def test_adamw_at_every_alignment(offset, gdt):
     assert ((m.double() - md).abs() <= mag * 2.0 ** -22).all()
     assert ((v.double() - vd).abs() <= vd * 2.0 ** -21).all()
     assert ((p.double() - want).abs() <= (want.abs() * 2.0 ** -8 + (p0.abs().double() + step.abs()) * 2.0 ** -18)).all()
+    ops.check_status()
+
+
+@pytest.mark.parametrize("pdt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("offset", [0, 8, 1])
+def test_adamw_update_is_correctly_rounded(pdt, offset):
+    """From a parameter of 0 without decay the stored value is the update itself. At the first step its factors are exact
+    in fp32, so from the stored moments it has to be, bit for bit, what IEEE square root, quotients and product give."""
+    torch.manual_seed(14)
+    n, lr, b1, b2, eps = 8 * 2 ** 16 + 3, 1e-2, 0.9, 0.95, 1e-8
+    flat = lambda t: torch.cat([t.new_zeros(offset), t])[offset:]   # noqa: E731
+    p, g, m = (flat(t) for t in (torch.zeros(n, device=DEV, dtype=pdt), torch.randn(n, device=DEV),
+                                 torch.randn(n, device=DEV) * 0.1))
+    v = flat(torch.randn(n, device=DEV).square() * 10.0 ** torch.randint(-12, 1, (n,), device=DEV))
+    ew.adamw_step_(p, g, m, v, lr=lr, beta1=b1, beta2=b2, eps=eps, weight_decay=0.0, step=1)
+    f = np.float32
+    root = np.sqrt(v.cpu().numpy()) / np.sqrt(f(1) - f(b2)) + f(eps)
+    want = -(f(lr) / (f(1) - f(b1)) * (m.cpu().numpy() / root))
+    assert want.dtype == f and torch.equal(p.cpu(), torch.from_numpy(want).to(pdt))
     ops.check_status()
 
 
