@@ -307,11 +307,8 @@ rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ src, int sr
 }
 
 // ------------------------------------------------------------------ SwiGLU
-// gu = [T, 2F] with gate in columns [0,F) and up in [F,2F); h = silu(gate) * up. Bound by memory (8192 x 14336: 0.172 ->
-// 0.113 ms, 6.2 TB/s) with 32-bit index divisions and the sigmoid as one exponential and one approximate reciprocal (2 ulp of fp32, 2^14 below the rounding
-// of the result).
-__device__ __forceinline__ float sigmoid_approx(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
-
+// gu = [T, 2F] with gate in columns [0,F) and up in [F,2F); h = silu(gate) * up. Bound by memory with 32-bit index
+// divisions (a 64-bit one costs more than the rest of the body).
 template <typename I>
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h, I total, int F) {
@@ -323,7 +320,7 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
     load8(gu + t * 2 * F + c, g);
     load8(gu + t * 2 * F + F + c, u);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = g[j] * sigmoid_approx(g[j]) * u[j];
+    for (int j = 0; j < 8; ++j) o[j] = g[j] / (1.f + __expf(-g[j])) * u[j];
     store8(h + t * F + c, o);
   }
 }
@@ -342,7 +339,7 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __r
     load8(dh + t * F + c, d);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float sg = sigmoid_approx(g[j]);
+      const float sg = 1.f / (1.f + __expf(-g[j]));
       const float silu = g[j] * sg;
       du[j] = d[j] * silu;
       dg[j] = d[j] * u[j] * (sg + silu * (1.f - sg));

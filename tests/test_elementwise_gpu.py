@@ -119,6 +119,24 @@ def test_cast_scale():
     torch.testing.assert_close(c, 1 + 2 * b.float())
 
 
+def test_swiglu_over_the_range_of_the_gate():
+    """Gates down to where the exponential nears the largest fp32 value (the quotient is tiny there, and not 0). Bound:
+    an argument of up to 88.5 in the fast exponential is good to 88.5 * 2^-23; one rounding to bf16."""
+    gate = torch.cat([torch.linspace(-88.5, 88.5, 355), torch.linspace(-2, 2, 45)]).bfloat16()
+    x = torch.stack([gate, torch.ones_like(gate)]).to(DEV).view(1, -1).requires_grad_()
+    h = ew.swiglu(x)
+    h.backward(torch.ones_like(h))
+    ops.check_status()
+    g = gate.double()
+    silu, sg = g * torch.sigmoid(g), torch.sigmoid(g)
+    rel = 2.0 ** -8 + 88.5 * 2.0 ** -23
+    for got, want in ((h[0], silu), (x.grad[0, 400:], silu)):
+        assert ((got.detach().double().cpu() - want).abs() <= want.abs() * rel).all()
+    # the gate's gradient is a difference of terms: their size counts
+    size = sg + silu.abs() * (1 - sg)
+    assert ((x.grad[0, :400].double().cpu() - (sg + silu * (1 - sg))).abs() <= size * rel).all()
+
+
 @pytest.mark.parametrize("offset", [0, 8, 1])
 @pytest.mark.parametrize("gdt", [torch.float32, torch.bfloat16])
 def test_adamw_at_every_alignment(offset, gdt):
