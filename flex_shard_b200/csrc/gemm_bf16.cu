@@ -1222,7 +1222,7 @@ static int gemm_pair_launch(const void* a, const void* b, void* d, const void* c
 // D_e = alpha * A_e . B_e^T + beta * C_e for `count` equal matrices, each operand a stack of row-major bf16 matrices back
 // to back (A [count, M, K] or, a_mn, [count, K, M]; B likewise; C and D [count, M, N], all rows packed). Contiguous
 // dimensions must be multiples of 8. symmetric: every D_e is symmetric (M == N); only its tiles on or above the diagonal
-// are computed, and mirrored. Returns FSB_ERR_TOO_LARGE where SM pairs cannot be used.
+// are computed, and mirrored. Returns FSB_ERR_TOO_LARGE where fsb_gemm_pairs_usable() is 0.
 //
 // Bound by the tensor cores for stacks of expert matrices, by latency for a stack of attention heads (a 192 x 1536
 // matrix is a single tile, so one grid takes the whole stack). A Muon step over 64 experts of 2816 x 2048 and of
@@ -1237,7 +1237,7 @@ FSB_API int fsb_gemm_bf16_batched(const void* a, const void* b, void* d, const v
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return FSB_ERR_BAD_ARG;
-  if (pair_clusters(dev) < 0) return FSB_ERR_TOO_LARGE;
+  if (!g_use_pairs_fwd() || pair_clusters(dev) < 0) return FSB_ERR_TOO_LARGE;
   const long long tm = (M + 2 * BM - 1) / (2 * BM), tn = (N + BN - 1) / BN;
   const int upper = symmetric && tm > 1;
   const long long tiles = (upper ? tm * (tm + 1) / 2 : tm * tn) * count;
@@ -1408,6 +1408,12 @@ static int g_use_pairs_value() { return g_use_pairs; }
 FSB_API int fsb_gemm_set_pair_mode(int on) {
   g_use_pairs = on;
   return FSB_OK;
+}
+// 1 where the kernels on SM pairs may be used: they fit the current device and are not switched off.
+FSB_API int fsb_gemm_pairs_usable() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return g_use_pairs != 0 && dev >= 0 && dev < 64 && pair_clusters(dev) > 0;
 }
 
 // All-gather -> GEMM in one kernel: D[M,N] = A[M,K] . W[N,K]^T where W is row-sharded over

@@ -35,6 +35,7 @@ def _ensure():
         _lib.declare("fsb_muon_scale", [vp, vp, i32, i64, i32, f32, vp])
         _lib.declare("fsb_muon_update", [vp, i32, vp, i64, f32, f32, vp])
         _lib.declare("fsb_muon_workspace_floats", [i64, i32])
+        _lib.declare("fsb_gemm_pairs_usable", [])
         _lib.declare("fsb_gemm_bf16_batched", [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, f32, i32, vp, vp])
         _declared = True
 
@@ -81,9 +82,13 @@ def _batched(a, b, out, M, N, K, *, a_t=False, b_t=False, c=None, alpha=1.0, bet
 
 def batched_ns_supported(x: torch.Tensor) -> bool:
     """Stacks of equal matrices whose dimensions are multiples of 8 (16-byte rows, which the copy engine needs) run every
-    product of an iteration as one launch over the whole stack."""
-    return (x.is_cuda and x.dim() == 3 and 1 < x.shape[0] <= 65535 and x.shape[1] % 8 == 0 and x.shape[2] % 8 == 0
-            and x.numel() > 0)
+    product of an iteration as one launch over the whole stack, where SM pairs can be used. Others take a matrix at a
+    time."""
+    if not (x.is_cuda and x.dim() == 3 and 1 < x.shape[0] <= 65535 and x.shape[1] % 8 == 0 and x.shape[2] % 8 == 0
+            and x.numel() > 0):
+        return False
+    _ensure()
+    return bool(_lib.load().fsb_gemm_pairs_usable())
 
 
 def ns_iterations_batched(x: torch.Tensor, steps: int = 5, coeffs=NS_COEFFS) -> torch.Tensor:

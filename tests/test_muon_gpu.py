@@ -172,3 +172,23 @@ def test_prepare_and_scale_of_a_stack_match_the_matrices_alone(E, rows, cols):
         torch.testing.assert_close(ws[e, 0], ws1[0, 0], rtol=1e-5, atol=0)
         torch.testing.assert_close(ws[e, 0], u1.float().square().sum(), rtol=1e-5, atol=0)
     ops.check_status()
+
+
+def test_stacks_without_sm_pairs_take_a_matrix_at_a_time():
+    """With the kernels on SM pairs switched off (or where they do not fit), a stack gives what its matrices give alone."""
+    from flex_shard_b200.ops import _lib
+
+    torch.manual_seed(10)
+    g = torch.randn(3, 128, 256, device="cuda")
+    lib = _lib.load()
+    assert ns.batched_ns_supported(g)
+    lib.fsb_gemm_set_pair_mode(0)
+    try:
+        assert not ns.batched_ns_supported(g)
+        out = ns.newton_schulz(g)
+        assert torch.equal(out, torch.stack([ns.newton_schulz(m) for m in g]))
+        with pytest.raises(RuntimeError):
+            ns._batched(out, out, torch.empty(3, 128, 128, device="cuda", dtype=out.dtype), 128, 128, 256)
+    finally:
+        lib.fsb_gemm_set_pair_mode(1)
+    ops.check_status()
