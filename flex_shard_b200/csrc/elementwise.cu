@@ -397,17 +397,16 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const long long* __rest
   }
 }
 
-// The same result with one read and one write of the logits: the row is held on chip between the passes,
-// its first `smem_vecs` 16-byte vectors in shared memory and the rest (up to CE_RV per thread) in registers.
-// While the row streams in, every thread keeps a running maximum and a sum of exponentials relative to it
-// (rescaled when the maximum grows), so the exponentials of the first pass hide under the loads; the block
-// then combines the (max, sum) pairs, and the final pass turns the resident row into gradients while the
-// stores drain. Bound by memory as long as an SM holds two rows or parts of rows, so that one loads while the other
-// stores. PAIR: a row too long for that is split between the two CTAs of a cluster, which exchange their (max, sum).
+// The same result with one read and one write of the logits: the row is held on chip between the passes, in shared
+// memory. While it streams in, every thread keeps a running maximum and a sum of exponentials relative to it (rescaled
+// when the maximum grows), so the exponentials of the first pass hide under the loads; the block then combines the
+// (max, sum) pairs, and the final pass turns the resident row into gradients while the stores drain. Bound by memory as
+// long as an SM holds two rows or parts of rows, so that one loads while the other stores. PAIR: a row too long for that
+// is split between the two CTAs of a cluster, which exchange their (max, sum) and keep the first `smem_vecs` 16-byte
+// vectors of a half in shared memory, the rest (up to CE_RV per thread) in registers.
 // 8192 x 128256 logits: 1.24 ms with a whole row to an SM, 1.06 ms in halves (4.0 TB/s).
 constexpr int CE_RV = 4;
-constexpr int CE_SMEM_VECS = 14336;        // 224 KB of the row in shared memory (one CTA per SM)
-constexpr int CE_SMEM_VECS_HALF = 7040;    // 110 KB (two CTAs per SM)
+constexpr int CE_SMEM_VECS = 7040;    // 110 KB (two CTAs per SM)
 template <bool PAIR>
 __global__ void __launch_bounds__(CE_THREADS, PAIR ? 2 : 1)
 cross_entropy_resident_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ target,
@@ -444,9 +443,10 @@ cross_entropy_resident_kernel(__nv_bfloat16* __restrict__ logits, const long lon
 #pragma unroll
     for (int j = 0; j < 8; ++j) s += exp2f(fmaf(f[j], L2E, mo));
   };
+  constexpr int RV = PAIR ? CE_RV : 0;
   uint4 rv[CE_RV];
 #pragma unroll
-  for (int k = 0; k < CE_RV; ++k) {
+  for (int k = 0; k < RV; ++k) {
     const int idx = smem_vecs + tid + k * CE_THREADS;
     rv[k] = idx < nvec ? g[idx] : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);   // -inf: adds nothing
   }
@@ -462,7 +462,7 @@ cross_entropy_resident_kernel(__nv_bfloat16* __restrict__ logits, const long lon
     take(a);
   }
 #pragma unroll
-  for (int k = 0; k < CE_RV; ++k)
+  for (int k = 0; k < RV; ++k)
     if (smem_vecs + tid + k * CE_THREADS < nvec) take(rv[k]);
   float mx = block_max<CE_THREADS>(m, red);
   float se = block_sum<CE_THREADS>(m == -INFINITY ? 0.f : s * exp2f((m - mx) * L2E), red);
@@ -499,7 +499,7 @@ cross_entropy_resident_kernel(__nv_bfloat16* __restrict__ logits, const long lon
   };
   for (i = tid; i < smem_vecs; i += CE_THREADS) grad(rowv[i], i);   // each thread reads back what it stored itself
 #pragma unroll
-  for (int k = 0; k < CE_RV; ++k) {
+  for (int k = 0; k < RV; ++k) {
     const int idx = smem_vecs + tid + k * CE_THREADS;
     if (idx < nvec) grad(rv[k], idx);
   }
@@ -857,47 +857,45 @@ FSB_API int fsb_cross_entropy(void* logits, const long long* target, float* loss
                               long long ld, float grad_scale, long long ignore_index,
                               cudaStream_t stream) {
   if (V % 8 != 0 || ld % 8 != 0) return FSB_ERR_BAD_ARG;
-  const int nvec = V / 8;
-  const int smem_vecs = nvec < CE_SMEM_VECS ? nvec : CE_SMEM_VECS;
-  const int half = (nvec + 1) / 2;
-  if ((reinterpret_cast<uintptr_t>(logits) & 15) == 0 && nvec > CE_SMEM_VECS_HALF && half <= CE_SMEM_VECS_HALF + CE_RV * CE_THREADS &&
-      T < (1ll << 30)) {
-    const int vecs = half < CE_SMEM_VECS_HALF ? half : CE_SMEM_VECS_HALF;
-    const size_t smem = static_cast<size_t>(vecs) * 16;
-    if (cudaFuncSetAttribute(cross_entropy_resident_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
-      return FSB_ERR_LAUNCH;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(2 * T), 1, 1);
-    cfg.blockDim = dim3(CE_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = 2;
-    at.val.clusterDim.y = 1;
-    at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, cross_entropy_resident_kernel<true>, static_cast<__nv_bfloat16*>(logits), target, loss, V, ld,
-                           grad_scale, ignore_index, vecs) != cudaSuccess) {
-      cudaGetLastError();
-      return FSB_ERR_LAUNCH;
-    }
-    return launch_ok();
-  }
-  if ((reinterpret_cast<uintptr_t>(logits) & 15) == 0 && nvec - smem_vecs <= CE_RV * CE_THREADS) {
-    // the row fits on chip: one read and one write
-    const size_t smem = static_cast<size_t>(smem_vecs) * 16;
+  const int nvec = V / 8, half = (nvec + 1) / 2;
+  const bool aligned = (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+  __nv_bfloat16* x = static_cast<__nv_bfloat16*>(logits);
+  if (aligned && nvec <= CE_SMEM_VECS) {
+    const size_t smem = static_cast<size_t>(nvec) * 16;
     if (cudaFuncSetAttribute(cross_entropy_resident_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(smem)) != cudaSuccess)
       return FSB_ERR_LAUNCH;
     cross_entropy_resident_kernel<false><<<static_cast<unsigned>(T), CE_THREADS, smem, stream>>>(
-        static_cast<__nv_bfloat16*>(logits), target, loss, V, ld, grad_scale, ignore_index, smem_vecs);
+        x, target, loss, V, ld, grad_scale, ignore_index, nvec);
     return launch_ok();
   }
+  static int pairs[64] = {0};   // clusters of the pair form that fit a device at once (-1: unusable)
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (aligned && half <= CE_SMEM_VECS + CE_RV * CE_THREADS && T < (1ll << 30) && dev >= 0 && dev < 64) {
+    if (pairs[dev] == 0) pairs[dev] = fsb_resident_pairs(cross_entropy_resident_kernel<true>, CE_THREADS, CE_SMEM_VECS * 16);
+    if (pairs[dev] > 0) {
+      const int vecs = half < CE_SMEM_VECS ? half : CE_SMEM_VECS;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(static_cast<unsigned>(2 * T), 1, 1);
+      cfg.blockDim = dim3(CE_THREADS, 1, 1);
+      cfg.dynamicSmemBytes = static_cast<size_t>(vecs) * 16;
+      cfg.stream = stream;
+      cudaLaunchAttribute at{};
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = 2;
+      at.val.clusterDim.y = 1;
+      at.val.clusterDim.z = 1;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      const cudaError_t err = cudaLaunchKernelEx(&cfg, cross_entropy_resident_kernel<true>, x, target, loss, V, ld, grad_scale,
+                                                 ignore_index, vecs);
+      const int rc = launch_ok();   // also clears the error of a launch that failed
+      return err == cudaSuccess ? rc : FSB_ERR_LAUNCH;
+    }
+  }
   cross_entropy_kernel<<<static_cast<unsigned>(T), CE_THREADS, 0, stream>>>(
-      static_cast<__nv_bfloat16*>(logits), target, loss, V, ld, grad_scale, ignore_index);
+      x, target, loss, V, ld, grad_scale, ignore_index);
   return launch_ok();
 }
 
