@@ -9,6 +9,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from . import _lib
 from ._lib import count_launch
@@ -38,6 +39,10 @@ def _write_grad(dy, tokens, out, accumulate: bool) -> None:
     count_launch(4)
 
 
+def _hooked(weight) -> bool:
+    return bool(weight._backward_hooks) or bool(getattr(weight, "_post_accumulate_grad_hooks", None))
+
+
 class _Embedding(torch.autograd.Function):
     @staticmethod
     def forward(ctx, tokens, weight):
@@ -50,13 +55,16 @@ class _Embedding(torch.autograd.Function):
         (tokens,), weight = ctx.saved_tensors, ctx.weight
         if not ctx.needs_input_grad[1]:
             return None, None
+        if torch.is_grad_enabled() or not _lib.plain(dy, tokens):
+            # a gradient that is differentiated again, or batched gradients: the operator that autograd knows
+            return None, torch.ops.aten.embedding_dense_backward(dy, tokens, weight.shape[0], -1, False)
         tokens = tokens.reshape(-1).contiguous()
         dy = dy.reshape(-1, dy.shape[-1]).contiguous()
         if dy.data_ptr() % 16:
             dy = dy.clone()
         main = getattr(weight, "main_grad", None)
         if (isinstance(main, torch.Tensor) and main.dtype == torch.float32 and main.is_contiguous()
-                and main.shape == weight.shape and main.data_ptr() % 16 == 0):
+                and main.shape == weight.shape and main.data_ptr() % 16 == 0 and not _hooked(weight)):
             _write_grad(dy, tokens, main, bool(getattr(weight, "main_grad_written", False)))
             weight.main_grad_written = True
             return None, None
@@ -66,8 +74,10 @@ class _Embedding(torch.autograd.Function):
 
 
 def embedding(tokens, weight):
-    """Rows ``tokens`` (any shape, int32 or int64) of ``weight`` [V, D]."""
-    if (weight.is_cuda and weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.shape[1] % 8 == 0
+    """Rows ``tokens`` (any shape, int32 or int64) of ``weight`` [V, D]. Forward-mode derivatives, the ``torch.func``
+    transforms, tensor subclasses and compilers take PyTorch's operator."""
+    if (_lib.plain(tokens, weight) and forward_ad._current_level < 0 and not torch.compiler.is_compiling()
+            and weight.is_cuda and weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.shape[1] % 8 == 0
             and 0 < weight.shape[1] <= 8192 and weight.shape[0] > 0 and 0 < tokens.numel() < 2 ** 31
             and tokens.device == weight.device and tokens.dtype in (torch.int32, torch.int64)):
         return _Embedding.apply(tokens, weight)
@@ -75,7 +85,9 @@ def embedding(tokens, weight):
 
 
 class TokenEmbedding(nn.Embedding):
-    """``nn.Embedding`` (without padding row, norm limit or sparse gradients) on ``embedding``."""
+    """``nn.Embedding`` (without padding row, norm limit or sparse gradients) on ``embedding``. Where the gathered weight
+    has a ``main_grad`` its gradient goes there and not through autograd (as with the products and norms of this library),
+    unless the weight has hooks."""
 
     def forward(self, tokens):
         return embedding(tokens, self.weight)

@@ -279,6 +279,43 @@ def test_embedding_gradient(T, V, D, kind, main):
     assert ((got[0].double() - want).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32])
+def test_embedding_under_the_transforms_of_autograd(dtype):
+    """What PyTorch's operator can do besides a backward pass: batched gradients, second derivatives, forward mode,
+    ``torch.func``, hooks on a weight whose gradient would go elsewhere. All sums here are exact."""
+    import torch.autograd.forward_ad as fwd
+
+    from flex_shard_b200.ops.embedding import TokenEmbedding, embedding
+
+    torch.manual_seed(13)
+    V, D = 11, 16
+    small = lambda *shape: torch.randint(-4, 5, shape, device=DEV).bfloat16()   # noqa: E731
+    tokens = torch.randint(0, V, (2, 3), device=DEV, dtype=dtype)
+    w = small(V, D).requires_grad_()
+    dys = small(4, 2, 3, D)
+    want = torch.stack([torch.zeros(V, D, device=DEV).index_add_(0, tokens.long().view(-1), d.float().view(-1, D))
+                        for d in dys]).bfloat16()
+    (got,) = torch.autograd.grad(embedding(tokens, w), w, dys, is_grads_batched=True)
+    assert torch.equal(got, want)
+    dy = dys[0].clone().requires_grad_()
+    (dw,) = torch.autograd.grad(embedding(tokens, w), w, dy, create_graph=True)
+    assert torch.equal(dw, want[0])
+    v = small(V, D)
+    assert torch.equal(torch.autograd.grad(dw, dy, v)[0], v[tokens.long()])
+    with fwd.dual_level():
+        y = embedding(tokens, fwd.make_dual(w.detach(), v))
+        assert torch.equal(fwd.unpack_dual(y).tangent, v[tokens.long()])
+    assert torch.equal(torch.func.grad(lambda t: (embedding(tokens, t) * dys[0]).sum())(w.detach()), want[0])
+    stack = torch.stack([w.detach(), v])
+    assert torch.equal(torch.vmap(embedding, in_dims=(None, 0))(tokens, stack), stack[:, tokens.long()])
+    m = TokenEmbedding(V, D, dtype=torch.bfloat16, device=DEV)
+    m.weight.main_grad, m.weight.main_grad_written, seen = torch.zeros(V, D, device=DEV), False, []
+    m.weight.register_hook(seen.append)
+    m(tokens).backward(dys[0])
+    assert torch.equal(seen[0], want[0]) and torch.equal(m.weight.grad, want[0]) and not m.weight.main_grad_written
+    ops.check_status()
+
+
 @pytest.mark.parametrize("V", [56320, 56328, 102400, 145408, 145416])
 def test_cross_entropy_of_rows_on_either_side_of_the_splits(V):
     """Rows of one CTA, of a pair of CTAs (odd halves, the largest) and too long to stay on chip; targets in both halves,
