@@ -2,11 +2,13 @@
 
 ``mla_operands`` rotates the rotary part of every query head, appends the rotated rotary key (one for all heads) to every
 head's own key part and separates the values, in one kernel forward and one backward (``csrc/mla.cu``). Tensors the
-kernel does not take (CPU, other dtypes, widths that are no multiple of 8) go through the same steps in PyTorch.
+kernel does not take (CPU, other dtypes, widths that are no multiple of 8) go through the same steps in PyTorch, as do
+forward-mode derivatives, the ``torch.func`` transforms, and gradients that are batched or differentiated again.
 """
 from __future__ import annotations
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib
 from ._lib import count_launch
@@ -37,6 +39,13 @@ def mla_operands_ref(q, kvb, k_pe, table, nope: int):
     return torch.cat([q_nope, q_pe], dim=-1), torch.cat([k_nope, k_pe.expand(B, S, H, rope)], dim=-1), v
 
 
+def _grads_ref(dquery, dkey, dvalue, table, nope: int):
+    """Gradients of the three inputs from PyTorch operations (a linear map, differentiable and batchable)."""
+    dk_pe = _rope_ref(dkey[..., nope:].float().sum(2, keepdim=True), table, True).squeeze(2)
+    return (torch.cat([dquery[..., :nope], _rope_ref(dquery[..., nope:], table, True)], dim=-1),
+            torch.cat([dkey[..., :nope], dvalue], dim=-1), dk_pe.to(dkey.dtype))
+
+
 class _MlaOperands(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, kvb, k_pe, table, nope):
@@ -58,6 +67,8 @@ class _MlaOperands(torch.autograd.Function):
     def backward(ctx, dquery, dkey, dvalue):
         (table,) = ctx.saved_tensors
         B, S, H, nope, rope, value = ctx.dims
+        if torch.is_grad_enabled() or not _lib.plain(dquery, dkey, dvalue):
+            return (*_grads_ref(dquery, dkey, dvalue, table, nope), None, None)
         dquery, dkey, dvalue = (g.contiguous() if g.data_ptr() % 16 == 0 else g.clone(memory_format=torch.contiguous_format)
                                 for g in (dquery, dkey, dvalue))
         dq = torch.empty_like(dquery)
@@ -72,6 +83,8 @@ class _MlaOperands(torch.autograd.Function):
 
 
 def _native(q, kvb, k_pe, table, nope) -> bool:
+    if not _lib.plain(q, kvb, k_pe, table) or forward_ad._current_level >= 0 or torch.compiler.is_compiling():
+        return False
     B, S, H, width = q.shape
     rope, value = width - nope, kvb.shape[-1] - nope
     return (q.is_cuda and all(t.dtype == torch.bfloat16 and t.device == q.device for t in (q, kvb, k_pe))

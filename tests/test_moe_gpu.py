@@ -102,6 +102,39 @@ def test_latent_attention_operands_match_the_torch_steps(B, S, H, nope, rope, va
     ops.check_status()
 
 
+def test_latent_attention_operands_under_the_transforms_of_autograd():
+    """Batched gradients, second derivatives and forward mode of what is a linear map of its inputs, against the torch
+    steps; the kernel's sum over heads is rounded once, theirs between heads."""
+    import torch.autograd.forward_ad as fwd
+
+    from flex_shard_b200.ops import elementwise as ew
+    from flex_shard_b200.ops import mla
+
+    torch.manual_seed(8)
+    dev = torch.device("cuda")
+    B, S, H, nope, rope, value = 2, 5, 3, 16, 8, 24
+    table = ew.rope_table(S, rope, 10000.0, dev)
+    shapes = [(B, S, H, nope + rope), (B, S, H, nope + value), (B, S, rope)]
+    rand = lambda *s: torch.randn(*s, device=dev).bfloat16()   # noqa: E731
+    xs, vs = [rand(*s).requires_grad_() for s in shapes], [rand(*s) for s in shapes]
+    dys = [rand(4, B, S, H, n) for n in (nope + rope, nope + rope, value)]
+    assert mla._native(*xs, table, nope)
+    close = lambda a, b: torch.testing.assert_close(a.float(), b.float(), rtol=2.0 ** -6, atol=H * 2.0 ** -6)   # noqa: E731
+    res = []
+    for fn in (mla.mla_operands, mla.mla_operands_ref):
+        outs = fn(*xs, table, nope)
+        batched = torch.autograd.grad(outs, xs, dys, is_grads_batched=True, retain_graph=True)
+        first = [d[0].clone().requires_grad_() for d in dys]
+        grads = torch.autograd.grad(outs, xs, first, create_graph=True)
+        second = torch.autograd.grad(grads, first, vs)
+        with fwd.dual_level():
+            ts = [fwd.unpack_dual(o).tangent for o in fn(*(fwd.make_dual(x.detach(), v) for x, v in zip(xs, vs)), table, nope)]
+        res.append([*batched, *grads, *second, *ts])
+    for a, b in zip(*res):
+        close(a, b)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("counts,D,F,dtype", [([0, 700, 1, 0, 513, 256, 1200, 0], 512, 320, torch.bfloat16),
                                               ([385, 130, 900, 0], 264, 640, torch.float32), ([3000], 256, 256, torch.bfloat16)])
 def test_grouped_products_on_sm_pairs(counts, D, F, dtype):
