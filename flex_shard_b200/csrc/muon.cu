@@ -47,12 +47,35 @@ __device__ __forceinline__ float block_sum_256(float acc, float* red) {
   return t;   // valid in thread 0
 }
 
+// Adds the blocks' sums of a matrix (blockIdx.y; ws is its workspace): the block that finishes last adds the partial sums
+// in index order, a fixed order whatever the schedule was.
+__device__ __forceinline__ void finish_sum(float acc, float* ws) {
+  __shared__ float red[8];
+  __shared__ int last;
+  const float t = block_sum_256(acc, red);
+  if (threadIdx.x == 0) {
+    ws[kWsHeader + blockIdx.x] = t;
+    __threadfence();
+    const unsigned prev = atomicAdd(reinterpret_cast<unsigned*>(ws + 1), 1u);
+    last = prev == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  float s = 0.f;
+  for (int i = threadIdx.x; i < static_cast<int>(gridDim.x); i += 256) s += __ldcg(ws + kWsHeader + i);
+  __syncthreads();
+  const float total = block_sum_256(s, red);
+  if (threadIdx.x == 0) {
+    ws[0] = total;
+    *reinterpret_cast<unsigned*>(ws + 1) = 0u;   // ready for the next use of the workspace
+  }
+}
+
 template <typename GT>
 __global__ void __launch_bounds__(256)
 muon_prepare_kernel(float* __restrict__ mom, const GT* __restrict__ g, __nv_bfloat16* __restrict__ u,
                     float* __restrict__ ws, long long n, float mu, int nesterov) {
-  __shared__ float red[8];
-  __shared__ int last;
   const long long tid = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   mom += blockIdx.y * n;
@@ -93,30 +116,42 @@ muon_prepare_kernel(float* __restrict__ mom, const GT* __restrict__ g, __nv_bflo
     const float ur = __bfloat162float(ub);
     acc += ur * ur;
   }
-  const float t = block_sum_256(acc, red);
-  if (threadIdx.x == 0) {
-    ws[kWsHeader + blockIdx.x] = t;
-    __threadfence();
-    const unsigned prev = atomicAdd(reinterpret_cast<unsigned*>(ws + 1), 1u);
-    last = prev == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  // the last block to finish: add the partials in index order (a fixed order whatever the schedule was)
-  float s = 0.f;
-  for (int i = threadIdx.x; i < static_cast<int>(gridDim.x); i += 256) s += __ldcg(ws + kWsHeader + i);
-  __syncthreads();
-  const float total = block_sum_256(s, red);
-  if (threadIdx.x == 0) {
-    ws[0] = total;
-    *reinterpret_cast<unsigned*>(ws + 1) = 0u;   // ready for the next use of the workspace
-  }
+  finish_sum(acc, ws);
 }
 
+// The squares of stacked bf16 matrices alone, in the order in which the prepare kernel adds them (for aligned matrices).
+__global__ void __launch_bounds__(256)
+muon_sum_squares_kernel(const __nv_bfloat16* __restrict__ u, float* __restrict__ ws, long long n) {
+  const long long tid = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+  u += blockIdx.y * n;
+  ws += blockIdx.y * (kWsHeader + gridDim.x);
+  float acc = 0.f;
+  long long done = 0;
+  if (aligned16(u)) {
+    const long long nv = n / 8;
+    for (long long i = tid; i < nv; i += stride) {
+      float v[8];
+      load8(u + i * 8, v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc += v[j] * v[j];
+    }
+    done = nv * 8;
+  }
+  for (long long i = done + tid; i < n; i += stride) {
+    const float v = __bfloat162float(u[i]);
+    acc += v * v;
+  }
+  finish_sum(acc, ws);
+}
+
+// DIVIDE: x / norm (stacks), correctly rounded, as PyTorch divides; else x * (1 / norm) (single matrices).
+template <bool DIVIDE>
 __global__ void __launch_bounds__(256)
 muon_scale_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ sumsq, int ws_stride, long long n, float eps) {
-  const float inv = 1.f / fmaxf(sqrtf(sumsq[static_cast<long long>(blockIdx.y) * ws_stride]), eps);
+  const float norm = fmaxf(sqrtf(sumsq[static_cast<long long>(blockIdx.y) * ws_stride]), eps);
+  const float inv = 1.f / norm;
+  auto scaled = [&](float v) { return DIVIDE ? v / norm : v * inv; };
   x += blockIdx.y * n;
   const long long tid = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -127,12 +162,12 @@ muon_scale_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ sumsq
       float v[8];
       load8(x + i * 8, v);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] *= inv;
+      for (int j = 0; j < 8; ++j) v[j] = scaled(v[j]);
       store8(x + i * 8, v);
     }
     done = nv * 8;
   }
-  for (long long i = done + tid; i < n; i += stride) x[i] = __float2bfloat16(__bfloat162float(x[i]) * inv);
+  for (long long i = done + tid; i < n; i += stride) x[i] = __float2bfloat16(scaled(__bfloat162float(x[i])));
 }
 
 template <typename PT>
@@ -165,16 +200,10 @@ inline int grid_for(long long n) {
 }
 }  // namespace
 
-// Blocks per matrix of a stack of `count` matrices of n elements: the whole stack shares the block budget.
-static int stack_grid(long long n, int count) {
-  const int most = kMaxBlocks / count > 0 ? kMaxBlocks / count : 1;
-  const int want = grid_for(n);
-  return want < most ? want : most;
-}
-
 // Floats a workspace for `count` matrices of n elements needs (it must be zero before its first use; a finished call
-// leaves it reusable for the same sizes). Matrix m's sum of squares is at m * (floats / count).
-FSB_API int fsb_muon_workspace_floats(long long n, int count) { return count * (kWsHeader + stack_grid(n, count)); }
+// leaves it reusable for the same sizes). Matrix m's sum of squares is at m * (floats / count). Every matrix of a stack has
+// the blocks that it would have alone, so its sum has the same bits whatever the stack holds.
+FSB_API int fsb_muon_workspace_floats(long long n, int count) { return count * (kWsHeader + grid_for(n)); }
 
 // mom, g, u: `count` matrices of n elements back to back; ws receives sum(u^2) of each. Bound by memory (12 bytes an
 // element): the stacks of 64 experts and two blocks' heads take 1.4 + 0.5 ms here and in the scale kernel, where PyTorch's
@@ -183,7 +212,7 @@ FSB_API int fsb_muon_prepare(float* mom, const void* g, int g_fp32, void* u, flo
                              float mu, int nesterov, cudaStream_t stream) {
   if (n <= 0 || count <= 0) return FSB_OK;
   if (count > 65535) return FSB_ERR_TOO_LARGE;
-  const dim3 grid(stack_grid(n, count), count);
+  const dim3 grid(grid_for(n), count);
   if (g_fp32)
     muon_prepare_kernel<float><<<grid, 256, 0, stream>>>(mom, static_cast<const float*>(g),
         static_cast<__nv_bfloat16*>(u), ws, n, mu, nesterov);
@@ -193,13 +222,24 @@ FSB_API int fsb_muon_prepare(float* mom, const void* g, int g_fp32, void* u, flo
   return cudaGetLastError() == cudaSuccess ? FSB_OK : FSB_ERR_LAUNCH;
 }
 
+// ws receives the sums of squares of `count` bf16 matrices of n elements back to back, as fsb_muon_prepare leaves them.
+FSB_API int fsb_muon_sum_squares(const void* u, float* ws, long long n, int count, cudaStream_t stream) {
+  if (n <= 0 || count <= 0) return FSB_OK;
+  if (count > 65535) return FSB_ERR_TOO_LARGE;
+  muon_sum_squares_kernel<<<dim3(grid_for(n), count), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(u), ws, n);
+  return cudaGetLastError() == cudaSuccess ? FSB_OK : FSB_ERR_LAUNCH;
+}
+
 // x: `count` matrices of n elements, each divided by its norm; ws_stride: floats between two matrices' sums of squares.
-FSB_API int fsb_muon_scale(void* x, const float* sumsq, int ws_stride, long long n, int count, float eps,
+// divide: a division per element, else one of the norm and a product per element.
+FSB_API int fsb_muon_scale(void* x, const float* sumsq, int ws_stride, long long n, int count, float eps, int divide,
                            cudaStream_t stream) {
   if (n <= 0 || count <= 0) return FSB_OK;
   if (count > 65535) return FSB_ERR_TOO_LARGE;
-  muon_scale_kernel<<<dim3(stack_grid(n, count), count), 256, 0, stream>>>(static_cast<__nv_bfloat16*>(x), sumsq,
-                                                                          ws_stride, n, eps);
+  const dim3 grid(grid_for(n), count);
+  __nv_bfloat16* xb = static_cast<__nv_bfloat16*>(x);
+  if (divide) muon_scale_kernel<true><<<grid, 256, 0, stream>>>(xb, sumsq, ws_stride, n, eps);
+  else muon_scale_kernel<false><<<grid, 256, 0, stream>>>(xb, sumsq, ws_stride, n, eps);
   return cudaGetLastError() == cudaSuccess ? FSB_OK : FSB_ERR_LAUNCH;
 }
 

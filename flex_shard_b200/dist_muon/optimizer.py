@@ -369,10 +369,11 @@ class DistMuon(torch.optim.Optimizer):
             k, n = len(mine), mine[0]
             blk = full[:k * n]
             stack = (blk.reshape(k, blk.shape[-2], blk.shape[-1]) if it.resolved.batch else blk.reshape(k, n, -1))
-            from ..ops.newton_schulz import batched_ns_supported
+            from ..ops.newton_schulz import batched_ns_supported, orthogonalise_stack_
 
             if batched_ns_supported(stack):
-                x = newton_schulz(stack, group["ns_steps"], group["ns_coefficients"], group["eps"])
+                x = orthogonalise_stack_(stack.to(torch.bfloat16, copy=True).contiguous(), group["ns_steps"],
+                                         group["ns_coefficients"], group["eps"])
                 out[:k * n].copy_(x.reshape(blk.shape))
                 return out
         pos = 0

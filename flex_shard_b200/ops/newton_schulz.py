@@ -32,7 +32,8 @@ def _ensure():
         c = ctypes
         vp, i32, i64, f32 = c.c_void_p, c.c_int, c.c_longlong, c.c_float
         _lib.declare("fsb_muon_prepare", [vp, vp, i32, vp, vp, i64, i32, f32, i32, vp])
-        _lib.declare("fsb_muon_scale", [vp, vp, i32, i64, i32, f32, vp])
+        _lib.declare("fsb_muon_sum_squares", [vp, vp, i64, i32, vp])
+        _lib.declare("fsb_muon_scale", [vp, vp, i32, i64, i32, f32, i32, vp])
         _lib.declare("fsb_muon_update", [vp, i32, vp, i64, f32, f32, vp])
         _lib.declare("fsb_muon_workspace_floats", [i64, i32])
         _lib.declare("fsb_gemm_pairs_usable", [])
@@ -158,10 +159,30 @@ def _normalise_cuda(x: torch.Tensor, eps: float) -> torch.Tensor:
     _ensure()
     x = x.contiguous().clone()
     ss = (x.float() ** 2).sum().reshape(1)
-    rc = _lib.load().fsb_muon_scale(x.data_ptr(), ss.data_ptr(), 1, x.numel(), 1, eps, _lib.stream_ptr(x.device))
+    return _normalise_(x, ss.view(1, 1), eps)
+
+
+def _normalise_(u: torch.Tensor, ws: torch.Tensor, eps: float) -> torch.Tensor:
+    """Divides every matrix of ``u`` by its norm in place, whose square is in ``ws[m, 0]`` (a workspace as ``_workspace``
+    gives it). Stacks divide element by element; a single matrix is multiplied by the norm's reciprocal."""
+    _ensure()
+    count = u.shape[0] if u.dim() == 3 else 1
+    rc = _lib.load().fsb_muon_scale(u.data_ptr(), ws.data_ptr(), ws.shape[1], u.numel() // count, count, eps,
+                                    int(u.dim() == 3), _lib.stream_ptr(u.device))
     _lib.check(rc, "fsb_muon_scale")
     count_launch()
-    return x
+    return u
+
+
+def _sum_squares(u: torch.Tensor) -> torch.Tensor:
+    """Workspace with the squared norms of the matrices of a contiguous bf16 stack: the bits that ``_prepare`` leaves
+    when it makes the stack (of matrices on 16-byte boundaries), however many matrices the stack has."""
+    _ensure()
+    ws = _workspace(u.device, u[0].numel(), u.shape[0])
+    rc = _lib.load().fsb_muon_sum_squares(u.data_ptr(), ws.data_ptr(), u[0].numel(), u.shape[0], _lib.stream_ptr(u.device))
+    _lib.check(rc, "fsb_muon_sum_squares")
+    count_launch()
+    return ws
 
 
 def _prepare(momentum, grad, mu, nesterov, count):
@@ -192,11 +213,17 @@ def muon_direction_(momentum: torch.Tensor, grad: torch.Tensor, mu: float, neste
         return _newton_schulz_cpu(u, steps, coeffs, eps)
     count = grad.shape[0] if grad.dim() == 3 else 1
     u, ws = _prepare(momentum, grad, mu, nesterov, count)
-    rc = _lib.load().fsb_muon_scale(u.data_ptr(), ws.data_ptr(), ws.shape[1], u.numel() // count, count, eps,
-                                    _lib.stream_ptr(u.device))
-    _lib.check(rc, "fsb_muon_scale")
-    count_launch()
-    return (ns_iterations_batched if grad.dim() == 3 else ns_iterations)(u, steps, coeffs)
+    if grad.dim() == 3:
+        return orthogonalise_stack_(u, steps, coeffs, eps, ws)
+    return ns_iterations(_normalise_(u, ws, eps), steps, coeffs)
+
+
+def orthogonalise_stack_(u: torch.Tensor, steps: int, coeffs, eps: float, ws: torch.Tensor | None = None) -> torch.Tensor:
+    """Approximate polar factors of a contiguous bf16 stack that ``batched_ns_supported`` accepts; overwrites ``u``. What a
+    stack that stays where it is stored (``ws``: the norms' workspace that its momentum kernel left) and matrices that
+    came over an exchange have in common, so that the number of ranks does not show in the bits."""
+    assert u.dtype == torch.bfloat16 and u.is_contiguous()
+    return ns_iterations_batched(_normalise_(u, _sum_squares(u) if ws is None else ws, eps), steps, coeffs)
 
 
 def muon_momentum_direction_(momentum: torch.Tensor, grad: torch.Tensor, mu: float, nesterov: bool) -> torch.Tensor:

@@ -157,20 +157,68 @@ def test_batched_products_of_any_size_stay_inside_their_matrix(E, rows, cols):
     ops.check_status()
 
 
-@pytest.mark.parametrize("E,rows,cols", [(3, 40, 72), (2, 5, 9), (1, 300, 700)])
+@pytest.mark.parametrize("E,rows,cols", [(3, 40, 72), (2, 5, 9), (1, 300, 700), (5, 1408, 4096)])
 def test_prepare_and_scale_of_a_stack_match_the_matrices_alone(E, rows, cols):
-    """One launch over a stack gives the bits of one launch per matrix, sums of squares included up to their order
-    (fp32 sums of at most 210 000 terms)."""
+    """One launch over a stack gives the bits of one launch per matrix, sums of squares included, whatever else the stack
+    holds (here matrices of very different norms); scaling divides every matrix by its own norm, rounded once to bf16."""
     torch.manual_seed(9)
-    g = torch.randn(E, rows, cols, device="cuda")
-    m = torch.randn(E, rows, cols, device="cuda")
+    size = 10.0 ** torch.arange(E, device="cuda").view(E, 1, 1)
+    g = torch.randn(E, rows, cols, device="cuda") * size
+    m = torch.randn(E, rows, cols, device="cuda") * size
     ms = m.clone()
     u, ws = ns._prepare(m, g, 0.95, True, E)
     for e in range(E):
         u1, ws1 = ns._prepare(ms[e], g[e], 0.95, True, 1)
         assert torch.equal(u[e], u1) and torch.equal(m[e], ms[e])
-        torch.testing.assert_close(ws[e, 0], ws1[0, 0], rtol=1e-5, atol=0)
-        torch.testing.assert_close(ws[e, 0], u1.float().square().sum(), rtol=1e-5, atol=0)
+        if (rows * cols) % 8 == 0:
+            assert torch.equal(ws[e, 0], ws1[0, 0])      # (matrices off the 16-byte grid are added in another order)
+        torch.testing.assert_close(ws[e, 0].double(), u1.double().square().sum(), rtol=1e-5, atol=0)
+    if (rows * cols) % 8 == 0:
+        assert torch.equal(ns._sum_squares(u)[:, 0], ws[:, 0])
+    norm = ws[:, 0].sqrt().view(E, 1, 1)
+    want = (u.float() / norm).bfloat16()
+    got = ns._normalise_(u.clone(), ws, 1e-7)
+    assert torch.equal(got, want)                        # the quotient in fp32, rounded once
+    ns._normalise_(u[0], ws[:1], 1e-7)                    # a matrix alone: times the reciprocal, two fp32 roundings more
+    torch.testing.assert_close(u[0].double(), want[0].double(), rtol=2.0 ** -7, atol=0)
+    assert (u[0] != want[0]).float().mean() < 0.01
+    ops.check_status()
+
+
+@pytest.mark.parametrize("E,rows,cols", [(4, 192, 1536), (3, 256, 128)])
+def test_stacks_have_the_same_direction_wherever_they_are_orthogonalised(E, rows, cols):
+    """Momentum, norm and iteration in one go (stacks that stay where they are stored) and in two steps around an
+    exchange (any part of a stack, the gradients' rows elsewhere) give the same bits."""
+    torch.manual_seed(11)
+    g, m = torch.randn(E, rows, cols, device="cuda"), torch.randn(E, rows, cols, device="cuda")
+    m2 = m.clone()
+    x = ns.muon_direction_(m, g, 0.95, True, 5)
+    u = ns.muon_momentum_direction_(m2, g, 0.95, True)
+    assert torch.equal(m, m2)
+    part = u[1:].clone()
+    assert torch.equal(x, ns.orthogonalise_stack_(u, 5, ns.NS_COEFFS, 1e-7))
+    assert torch.equal(x[1:], ns.orthogonalise_stack_(part, 5, ns.NS_COEFFS, 1e-7))
+    ops.check_status()
+
+
+def test_redistributed_stacks_take_the_shared_arithmetic():
+    """The computing stage of redistributed parameters gives a stack the direction it would have where it is stored."""
+    from types import SimpleNamespace
+
+    from flex_shard_b200.dist_muon import DistMuon
+
+    torch.manual_seed(12)
+    g = torch.randn(3, 64, 128, device="cuda")
+    opt = DistMuon([torch.nn.Parameter(torch.zeros(3, 64, 128, device="cuda"))], param_names=["experts"], lr=0.02)
+    group = opt.param_groups[0]
+    m = torch.zeros_like(g)
+    want = ns.muon_direction_(m.clone(), g, group["momentum"], group["nesterov"], group["ns_steps"],
+                              group["ns_coefficients"], group["eps"])
+    u = ns.muon_momentum_direction_(m, g, group["momentum"], group["nesterov"])
+    plan = SimpleNamespace(matrices=[(i, i + 1, 0) for i in range(3)])
+    kept = u.clone()
+    got = opt._compute(SimpleNamespace(resolved=SimpleNamespace(batch=True)), plan, u)
+    assert torch.equal(got, want) and torch.equal(u, kept)
     ops.check_status()
 
 
