@@ -1,7 +1,7 @@
 """Token embedding whose weight gradient is written once, into the reduction bucket where the weight has one.
 
 The forward is PyTorch's gather. The backward (``csrc/embedding.cu``) adds the output gradients of equal tokens in fp32 and
-in token order, straight into the weight's ``main_grad`` view or a new gradient. Other weights (CPU, other dtypes, widths)
+in an order that only the tokens decide, straight into the weight's ``main_grad`` view or a new gradient. Other weights (CPU, other dtypes, widths)
 take PyTorch's backward.
 """
 from __future__ import annotations
@@ -24,6 +24,8 @@ def _ensure():
 
         vp, i32, i64 = c.c_void_p, c.c_int, c.c_longlong
         _lib.declare("fsb_embedding_grad", [vp, vp, i32, i64, i32, i32, vp, i32, i32, vp, vp])
+        _lib.declare("fsb_embedding_scratch_ints", [i64, i32, i32])
+        _lib.load().fsb_embedding_scratch_ints.restype = i64
         _declared = True
 
 
@@ -31,12 +33,13 @@ def _write_grad(dy, tokens, out, accumulate: bool) -> None:
     _ensure()
     V, D = out.shape
     T = tokens.numel()
-    scratch = torch.empty(3 * V + T + 1, dtype=torch.int32, device=dy.device)
-    rc = _lib.load().fsb_embedding_grad(dy.data_ptr(), tokens.data_ptr(), int(tokens.dtype == torch.int64), T, V, D,
+    lib = _lib.load()
+    scratch = torch.empty(lib.fsb_embedding_scratch_ints(T, V, D), dtype=torch.int32, device=dy.device)
+    rc = lib.fsb_embedding_grad(dy.data_ptr(), tokens.data_ptr(), int(tokens.dtype == torch.int64), T, V, D,
                                         out.data_ptr(), int(out.dtype == torch.float32), int(accumulate),
                                         scratch.data_ptr(), _lib.stream_ptr(dy.device))
     _lib.check(rc, "fsb_embedding_grad")
-    count_launch(4)
+    count_launch(6 if T > 64 else 4)
 
 
 def _hooked(weight) -> bool:

@@ -279,6 +279,37 @@ def test_embedding_gradient(T, V, D, kind, main):
     assert ((got[0].double() - want).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("counts,V", [([64, 65, 63, 1], 9), ([2048, 2049, 128, 3], 5000), ([70000, 100, 65], 300), ([65], 1)])
+@pytest.mark.parametrize("main", [None, True])
+def test_embedding_gradient_of_frequent_tokens(counts, V, main):
+    """Values on either side of what one block adds (64 rows), of what it orders at once (2048 positions) and far above,
+    with others never read: the same bits on every run, and as good as a sum in fp32."""
+    from flex_shard_b200.ops.embedding import embedding
+
+    torch.manual_seed(15)
+    D, T = 40, sum(counts)
+    values = torch.linspace(0, V - 1, len(counts)).long()
+    tokens = torch.repeat_interleave(values, torch.tensor(counts))[torch.randperm(T)].to(DEV)
+    w = torch.randn(V, D, device=DEV).bfloat16().requires_grad_()
+    dy, base, got = torch.randn(T, D, device=DEV).bfloat16(), torch.randn(V, D, device=DEV), []
+    for _ in range(2):
+        w.grad = None
+        if main is not None:
+            w.main_grad, w.main_grad_written = base.clone(), main
+        embedding(tokens, w).backward(dy)
+        got.append(w.grad if main is None else w.main_grad)
+    assert torch.equal(*got)
+    want = torch.zeros(V, D, device=DEV, dtype=torch.float64).index_add_(0, tokens, dy.double())
+    mag = torch.zeros_like(want).index_add_(0, tokens, dy.double().abs())
+    if main:
+        want, mag = want + base, mag + base.abs()
+    # at most 64 additions, then one per 64 of them
+    n = 64 + max(counts) / 64 + 2
+    bound = mag * (n * 2.0 ** -24) + (want.abs() * 2.0 ** -8 if main is None else 0)
+    assert ((got[0].double() - want).abs() <= bound).all()
+    ops.check_status()
+
+
 @pytest.mark.parametrize("dtype", [torch.int64, torch.int32])
 def test_embedding_under_the_transforms_of_autograd(dtype):
     """What PyTorch's operator can do besides a backward pass: batched gradients, second derivatives, forward mode,
