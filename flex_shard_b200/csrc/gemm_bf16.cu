@@ -1287,11 +1287,20 @@ FSB_API int fsb_gemm_bf16_grouped(const void* a, const void* b, void* d, int mod
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return FSB_ERR_BAD_ARG;
-  // SM pairs where their 256 x 256 tiles are mostly full: row groups of two 128-row tiles or more on average, outputs of
-  // at least one tile per group. Eight products of 64 experts (49152 rows, 2816 x 2048 and 2048 x 1408): 3.16 ms on single
-  // SMs, 2.84 on pairs.
+  // SM pairs where their 256 x 256 tiles win against 128 x 256 per SM, measured on 8 to 64 groups of even and of uneven
+  // sizes (time on single SMs / on pairs). max_rows is the groups' rows plus 128 per group.
+  // Rows in groups (mode 1): a group's last tile is half empty when it has an odd number of 128-row tiles, and the
+  // epilogue of a pair's tile weighs more on a short contraction. From 640 rows a group at a depth of 1024 and more: 0.97
+  // to 1.3 (64 groups of 2816 x 2048, 768 rows: 493 / 474 us); 576 rows 0.90-1.16, 300 rows 0.78-1.09; depth 768
+  // 0.93-1.13, depth 512 0.66-1.1.
+  // Contraction over the groups' rows (mode 2): with few rows a tile is mostly epilogue. bf16 from 640 rows: 0.98-1.35;
+  // 576 rows 0.83-1.13, 300 rows 0.65-0.91. fp32 from 1500 rows: 1.02-1.27; 1024 rows 0.89-1.17, 640 rows 0.90-1.05;
+  // added to fp32, 2048 rows: 0.96-1.07. Heights that leave a tenth of the 256-row tiles empty lose (640 x 512: 0.85-1.0).
+  const long long depth = static_cast<long long>(max_rows) / (BM * (num_groups > 0 ? num_groups : 1));   // 1 + rows / 128
+  const long long padded_m = (static_cast<long long>(M) + 2 * BM - 1) / (2 * BM) * (2 * BM);
   const bool pairs = g_use_pairs_fwd() && num_groups <= MAX_GROUPS2 && N >= BN && pair_clusters(dev) > 0 &&
-                     (mode == 1 ? max_rows >= 3ll * BM * num_groups : M >= 2 * BM);
+                     (mode == 1 ? depth >= 6 && K >= 1024
+                                : !accumulate && depth >= (d_fp32 ? 12 : 6) && 10 * padded_m <= 11ll * M);
   if (mode == 1) {
     // A [max_rows, K] K-major; B stacked over experts
     rc = fsb_make_tmap_2d(&map_a, a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, max_rows, K, lda, BM, BK);

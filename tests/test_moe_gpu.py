@@ -164,3 +164,42 @@ def test_grouped_products_on_sm_pairs(counts, D, F, dtype):
         for got, ref, mag in pairs:
             bound = mag * (1280 * 2.0 ** -24) + ref.abs() * (2.0 ** -8 if got.dtype == torch.bfloat16 else 0)
             assert ((got.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("counts,D,F,dtype", [([1500, 0, 130, 2400, 901], 1032, 1248, torch.bfloat16),
+                                              ([640] * 4, 1024, 1024, torch.bfloat16), ([639] * 4, 1024, 1024, torch.bfloat16),
+                                              ([3000, 129, 1700], 264, 1248, torch.float32)])
+@pytest.mark.parametrize("pairs", [1, 0])
+def test_grouped_products_either_way(counts, D, F, dtype, pairs):
+    """Sizes at which the rule takes SM pairs (and just does not), on pairs and with pairs switched off: groups that end
+    in half a pair tile, an empty one, ragged widths; fp32 destinations written anew. Sums of n products in fp32."""
+    from flex_shard_b200.ops import _lib
+
+    torch.manual_seed(4)
+    dev = torch.device("cuda")
+    E = len(counts)
+    idx = torch.cat([torch.full((c,), e) for e, c in enumerate(counts)])[torch.randperm(sum(counts))].view(-1, 1).to(dev)
+    plan = moe.plan_routes(idx, E)
+    x = moe.moe_dispatch(torch.randn(idx.shape[0], D, device=dev).bfloat16(), plan).requires_grad_()
+    w = torch.randn(E, F, D, device=dev).bfloat16().requires_grad_()
+    if dtype == torch.float32:
+        w.main_grad, w.main_grad_written = torch.full((E, F, D), 7.0, device=dev), False
+    offs = plan.offs.tolist()
+    dy = torch.zeros(plan.max_rows, F, device=dev, dtype=torch.bfloat16)
+    dy[:offs[-1]] = torch.randn(offs[-1], F, device=dev).bfloat16()
+    lib = _lib.load()
+    lib.fsb_gemm_set_pair_mode(pairs)
+    try:
+        y = moe.grouped_linear(x, w, plan)
+        y.backward(dy)
+    finally:
+        lib.fsb_gemm_set_pair_mode(1)
+    ops.check_status()
+    dw = w.main_grad if dtype == torch.float32 else w.grad
+    for e in range(E):
+        r = slice(offs[e], offs[e + 1])
+        xe, we, de = x.detach()[r].double(), w.detach()[e].double(), dy[r].double()
+        for got, ref, mag, n in ((dw[e], de.t() @ xe, de.abs().t() @ xe.abs(), max(counts)),
+                                 (y[r], xe @ we.t(), xe.abs() @ we.abs().t(), D), (x.grad[r], de @ we, de.abs() @ we.abs(), F)):
+            bound = mag * (n * 2.0 ** -24) + ref.abs() * (2.0 ** -8 if got.dtype == torch.bfloat16 else 0)
+            assert ((got.double() - ref).abs() <= bound).all()
