@@ -404,7 +404,9 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const long long* __rest
 // long as an SM holds two rows or parts of rows, so that one loads while the other stores. PAIR: a row too long for that
 // is split between the two CTAs of a cluster, which exchange their (max, sum) and keep the first `smem_vecs` 16-byte
 // vectors of a half in shared memory, the rest (up to CE_RV per thread) in registers.
-// 8192 x 128256 logits: 1.24 ms with a whole row to an SM, 1.06 ms in halves (4.0 TB/s).
+// Rows of up to CE_SMEM_VECS vectors fit an SM twice (4096 x 56320: 208 us, 4.4 TB/s; 273 us with one row to an SM at a
+// time). Longer ones, a whole row to an SM against halves, 4096 rows: 56328 logits 273 / 280 us, 65536 294 / 292, 80000
+// 362 / 349, 102400 426 / 413, 128256 511 / 497, 145408 (past what an SM holds) 751 / 548.
 constexpr int CE_RV = 4;
 constexpr int CE_SMEM_VECS = 7040;    // 110 KB (two CTAs per SM)
 template <bool PAIR>
@@ -917,7 +919,6 @@ FSB_API int fsb_segment_op_host(const void* host_descs, int nseg, int blocks_per
   return launch_ok();
 }
 
-// step >= 1. p_fp32 / g_fp32 select the master and gradient dtypes.
 FSB_API int fsb_scale_by_scalar(void* x, const float* scale, long long n, cudaStream_t stream) {
   if ((reinterpret_cast<uintptr_t>(x) & 15) != 0) return FSB_ERR_BAD_ARG;
   if (n <= 0) return FSB_OK;
@@ -925,6 +926,7 @@ FSB_API int fsb_scale_by_scalar(void* x, const float* scale, long long n, cudaSt
   return launch_ok();
 }
 
+// step >= 1. p_fp32 / g_fp32 select the master and gradient dtypes.
 FSB_API int fsb_adamw(void* p, const void* g, float* m, float* v, void* p_lowp, long long n,
                       int p_fp32, int g_fp32, float lr, float beta1, float beta2, float eps,
                       float weight_decay, int step, float grad_scale, cudaStream_t stream) {
