@@ -1,8 +1,8 @@
 """Token embedding whose weight gradient is written once, into the reduction bucket where the weight has one.
 
-The forward is PyTorch's gather. The backward (``csrc/embedding.cu``) adds the output gradients of equal tokens in fp32 and
-in an order that only the tokens decide, straight into the weight's ``main_grad`` view or a new gradient. Other weights (CPU, other dtypes, widths)
-take PyTorch's backward.
+The forward is PyTorch's gather. The backward (``csrc/embedding.cu``) adds the output gradients of equal tokens in fp32,
+in an order that only the tokens decide, straight into the weight's ``main_grad`` view or a new gradient. Other weights
+(CPU, other dtypes, widths) take PyTorch's backward.
 """
 from __future__ import annotations
 
@@ -88,9 +88,11 @@ def embedding(tokens, weight):
 
 
 class TokenEmbedding(nn.Embedding):
-    """``nn.Embedding`` (without padding row, norm limit or sparse gradients) on ``embedding``. Where the gathered weight
-    has a ``main_grad`` its gradient goes there and not through autograd (as with the products and norms of this library),
-    unless the weight has hooks."""
+    """``nn.Embedding`` on ``embedding``; with a padding row, a norm limit, scaling by frequency or sparse gradients, PyTorch's.
+    Where the gathered weight has a ``main_grad`` its gradient goes there and not through autograd (as with the products and
+    norms of this library), unless the weight has hooks."""
 
     def forward(self, tokens):
+        if self.padding_idx is not None or self.max_norm is not None or self.scale_grad_by_freq or self.sparse:
+            return super().forward(tokens)
         return embedding(tokens, self.weight)

@@ -449,3 +449,23 @@ def test_a_gradient_does_not_keep_a_larger_tensor_alive(monkeypatch):
     m(torch.zeros(60, 8).bfloat16()).backward(torch.ones(64, 8).bfloat16())
     g = m.w.grad
     assert g.untyped_storage().nbytes() == g.numel() * g.element_size()
+
+
+def test_token_embedding_keeps_the_options_of_the_module():
+    """Options set on a model's embedding (a padding row, a norm limit, scaling by frequency, sparse gradients) act as on
+    ``nn.Embedding``."""
+    from flex_shard_b200.ops.embedding import TokenEmbedding
+
+    torch.manual_seed(0)
+    tokens = torch.tensor([[0, 2, 2, 1]])
+    for name, value in (("padding_idx", 2), ("max_norm", 0.5), ("scale_grad_by_freq", True), ("sparse", True)):
+        ours, ref = TokenEmbedding(4, 8), nn.Embedding(4, 8)
+        ref.load_state_dict(ours.state_dict())
+        for m in (ours, ref):
+            setattr(m, name, value)
+        a, b = ours(tokens), ref(tokens)
+        (a * torch.arange(8.0)).sum().backward()
+        (b * torch.arange(8.0)).sum().backward()
+        assert torch.equal(a, b) and torch.equal(ours.weight, ref.weight), name
+        assert ours.weight.grad.is_sparse == ref.weight.grad.is_sparse, name
+        assert torch.equal(ours.weight.grad.to_dense(), ref.weight.grad.to_dense()), name
