@@ -441,7 +441,7 @@ cross_entropy_resident_kernel(__nv_bfloat16* __restrict__ logits, const long lon
       s *= exp2f((m - vm) * L2E);
       m = vm;
     }
-    const float mo = -m * L2E;
+    const float mo = m == -INFINITY ? 0.f : -m * L2E;   // masked logits alone add exp2(-inf) = 0
 #pragma unroll
     for (int j = 0; j < 8; ++j) s += exp2f(fmaf(f[j], L2E, mo));
   };

@@ -231,6 +231,30 @@ def test_cross_entropy_gradient_of_a_scaled_loss(shape, factor):
     ops.check_status()
 
 
+@pytest.mark.parametrize("V", [1000, 56320, 102400, 133120, 145416])
+def test_cross_entropy_of_masked_logits(V):
+    """Logits of -inf: a whole row but one, either half, the first groups of eight, every other group."""
+    torch.manual_seed(16)
+    x = torch.randn(6, V, device=DEV).bfloat16()
+    tgt = torch.tensor([V // 2, V - 1, 3, V - 2, 8, V - 8], device=DEV)
+    x[0, :] = -torch.inf
+    x[0, V // 2] = 1.0
+    x[1, : V // 2] = -torch.inf
+    x[2, V // 2:] = -torch.inf
+    x[3, : V - 16] = -torch.inf
+    x[4].view(-1, 8)[::2] = -torch.inf
+    x[5, : V - 8] = -torch.inf
+    ref = x.double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(ref, tgt)
+    want.backward()
+    leaf = x.clone().requires_grad_()
+    loss = ew.cross_entropy(leaf * 1.0, tgt)
+    loss.backward()
+    assert abs(float(loss.detach()) - float(want.detach())) <= 1e-5 * abs(float(want.detach()))
+    torch.testing.assert_close(leaf.grad.double(), ref.grad, rtol=2.0 ** -8 + 2e-5, atol=1e-9)
+    ops.check_status()
+
+
 def test_cross_entropy_takes_batched_loss_gradients():
     torch.manual_seed(3)
     x, target = torch.randn(5, 1000, device=DEV).bfloat16(), torch.randint(0, 1000, (5,), device=DEV)
