@@ -236,7 +236,8 @@ FSB_API int fsb_muon_scale(void* x, const float* sumsq, int ws_stride, long long
                            cudaStream_t stream) {
   if (n <= 0 || count <= 0) return FSB_OK;
   if (count > 65535) return FSB_ERR_TOO_LARGE;
-  const dim3 grid(grid_for(n), count);
+  const int most = kMaxBlocks / count > 0 ? kMaxBlocks / count : 1;   // no sums here: the stack shares one grid's blocks
+  const dim3 grid(grid_for(n) < most ? grid_for(n) : most, count);
   __nv_bfloat16* xb = static_cast<__nv_bfloat16*>(x);
   if (divide) muon_scale_kernel<true><<<grid, 256, 0, stream>>>(xb, sumsq, ws_stride, n, eps);
   else muon_scale_kernel<false><<<grid, 256, 0, stream>>>(xb, sumsq, ws_stride, n, eps);
