@@ -572,7 +572,8 @@ __device__ __forceinline__ void adamw_update(float& pv, float gv, float& mv, flo
 // 8 elements per thread per iteration; `n8` full groups, then a scalar tail. Bound by memory (16 B of moments plus
 // parameter and gradient per element) as long as the SM clock is high; at the clocks of a training step the IEEE square
 // root and quotients, some 40 instructions an element, take about as long. WIDE: the fp32 arrays start on 32-byte
-// boundaries (every flat bucket does) and move in 32-byte accesses; otherwise 16-byte ones.
+// boundaries (every flat bucket does) and move in 32-byte accesses; otherwise 16-byte ones. 268 M parameters with an fp32
+// gradient: 1.16 ms in 16-byte accesses, 1.02 in 32-byte ones (6.3 TB/s).
 template <typename PT, typename GT, bool WIDE>
 __global__ void __launch_bounds__(256)
 adamw_kernel(PT* __restrict__ p, const GT* __restrict__ g, float* __restrict__ m,

@@ -117,6 +117,9 @@ def test_dist_muon_steps_a_stack_of_equal_matrices_in_one_go():
             launches.append(ops.launch_count() - before)
     for i, p in enumerate(singles):
         torch.testing.assert_close(stacked.detach()[i], p.detach(), rtol=0, atol=2e-3)
+        # and the steps themselves: two directions, each within 1e-2 of the matrix's own (as above)
+        moved, alone = stacked.detach()[i] - w[i], p.detach() - w[i]
+        assert (moved - alone).norm() <= 1e-2 * alone.norm()
     assert launches[0] * 3 < launches[1]            # 1 + 15 + 1 launches (plus normalisation) against 6 x 18
     ops.check_status()
 
