@@ -50,7 +50,9 @@ class _Embedding(torch.autograd.Function):
     @staticmethod
     def forward(ctx, tokens, weight):
         ctx.save_for_backward(tokens)
-        ctx.weight = weight      # its gradient destination is looked up when the gradient is there; its values are not needed
+        # a parameter's gradient destination is looked up when the gradient is there; a weight's values are not needed
+        ctx.weight = weight if weight.is_leaf else None
+        ctx.shape = weight.shape
         return F.embedding(tokens, weight)
 
     @staticmethod
@@ -60,18 +62,18 @@ class _Embedding(torch.autograd.Function):
             return None, None
         if torch.is_grad_enabled() or not _lib.plain(dy, tokens):
             # a gradient that is differentiated again, or batched gradients: the operator that autograd knows
-            return None, torch.ops.aten.embedding_dense_backward(dy, tokens, weight.shape[0], -1, False)
+            return None, torch.ops.aten.embedding_dense_backward(dy, tokens, ctx.shape[0], -1, False)
         tokens = tokens.reshape(-1).contiguous()
         dy = dy.reshape(-1, dy.shape[-1]).contiguous()
         if dy.data_ptr() % 16:
             dy = dy.clone()
         main = getattr(weight, "main_grad", None)
         if (isinstance(main, torch.Tensor) and main.dtype == torch.float32 and main.is_contiguous()
-                and main.shape == weight.shape and main.data_ptr() % 16 == 0 and not _hooked(weight)):
+                and main.shape == ctx.shape and main.data_ptr() % 16 == 0 and not _hooked(weight)):
             _write_grad(dy, tokens, main, bool(getattr(weight, "main_grad_written", False)))
             weight.main_grad_written = True
             return None, None
-        dw = torch.empty(weight.shape, dtype=weight.dtype, device=weight.device)
+        dw = torch.empty(ctx.shape, dtype=dy.dtype, device=dy.device)
         _write_grad(dy, tokens, dw, False)
         return None, dw
 

@@ -469,3 +469,17 @@ def test_token_embedding_keeps_the_options_of_the_module():
         assert torch.equal(a, b) and torch.equal(ours.weight, ref.weight), name
         assert ours.weight.grad.is_sparse == ref.weight.grad.is_sparse, name
         assert torch.equal(ours.weight.grad.to_dense(), ref.weight.grad.to_dense()), name
+
+
+def test_token_embedding_does_not_keep_a_temporary_weight():
+    """The gather needs no weight in its backward: a cast or otherwise computed one is freed after the forward."""
+    import weakref
+
+    from flex_shard_b200.ops.embedding import _Embedding
+
+    w = torch.randn(4, 8, requires_grad=True)
+    cast = w.bfloat16()
+    gone = weakref.ref(cast.untyped_storage())
+    y = _Embedding.apply(torch.tensor([0, 2]), cast)
+    del cast
+    assert gone() is None and y.requires_grad
